@@ -4,6 +4,7 @@
 // Per iteration (realworld/polar_gpu.py:100-125):
 //   mk_spmm   v = (M + tau_0 I) d, partial d.v per CTA; the last CTA to finish reduces
 //             the partials in a fixed order and writes a = rr / d.v
+//   mk_added  (operators with many added edges) their terms of v and d.v, then a
 //   mk_resid  r <- r - a v, r on the active rows -> history slot, partial r.r; the last
 //             CTA computes beta, chi and convergence for every column
 //   mk_dir    zeta recurrences / tracker / freezing for all (pole, column) items and the
@@ -34,8 +35,8 @@
 namespace polar {
 
 // ctl: [0] status [1] err [2] where [3] any [4] ran [5] nsteps [6] first
-//      [7] cnt_init [8] cnt_spmm [9] cnt_resid [10] cnt_dir [11] cnt_flush
-enum { C_STATUS = 0, C_ERR, C_WHERE, C_ANY, C_RAN, C_NSTEPS, C_FIRST, C_CNT0, C_CNT1, C_CNT3, C_CNT4, C_CNT5 };
+//      [7] cnt_init [8] cnt_spmm [9] cnt_resid [10] cnt_dir [11] cnt_flush [12] cnt_added
+enum { C_STATUS = 0, C_ERR, C_WHERE, C_ANY, C_RAN, C_NSTEPS, C_FIRST, C_CNT0, C_CNT1, C_CNT3, C_CNT4, C_CNT5, C_CNTX };
 
 POLAR_D bool last_cta(int* cnt) {
   __shared__ int s_last;
@@ -105,7 +106,8 @@ __global__ void __launch_bounds__(kBlock) mk_init(const __grid_constant__ SolveP
 }
 
 // ---- edges added by the greedy (Op.add): v += sum_S w b b^T d, d.v += d^T (that) ------------
-// Run by the SpMM's last CTA after every row of v is final.  Thread item = (added-edge
+// Run by the SpMM's last CTA after every row of v is final, for a few edges; mk_added below
+// takes longer lists.  Thread item = (added-edge
 // row, column); each row's change is its own term w (d_r - d_k) summed over its added
 // neighbours in list order, and the d.v correction x_r (v_new - v_old) is summed per column
 // over the rows in a fixed order in `tmp` (shared, kWarps * kMaxLd doubles).
@@ -142,6 +144,24 @@ POLAR_D void apply_added_edges(const SolvePrm<T>& P, double* tmp, double* s_col)
   __syncthreads();
   if (threadIdx.x < ld) s_col[threadIdx.x] += colsum;
   __syncthreads();
+}
+
+// Added edges go to mk_added when the SpMM's last CTA would need more than one pass of its
+// threads over the (row, column) items; up to that its tail is shorter than one more launch.
+template <typename T>
+POLAR_HD bool added_split(const SolvePrm<T>& P) {
+  return (long long)P.g.nx * P.ld > kBlock;
+}
+
+// a = rr / d.v per column, from the complete d.v (one CTA).
+template <typename T>
+POLAR_D void step_length(const SolvePrm<T>& P, const double* dv) {
+  for (int c = threadIdx.x; c < P.ld; c += blockDim.x) {
+    const int a_on = P.act[c];
+    const double a = a_on ? P.rr[c] / dv[c] : 0.0;
+    if (a_on && !isfinite(a)) atomicCAS(P.ctl + C_ERR, 0, (int)POLAR_ERR_NONFINITE);
+    P.ag[c] = a;
+  }
 }
 
 // ---- v = (M + tau_0 I) d and d.v -------------------------------------------------------
@@ -321,13 +341,62 @@ __global__ void __launch_bounds__(kBlock, POLAR_SPMM_MINB) mk_spmm(const __grid_
       for (int c = threadIdx.x; c < ld; c += blockDim.x) s_col[c] = s_h[c] + s_col[c];
       __syncthreads();
     }
-    if (g.nx > 0) apply_added_edges(P, red, s_col);
-    for (int c = threadIdx.x; c < ld; c += blockDim.x) {
-      const int a_on = P.act[c];
-      const double a = a_on ? P.rr[c] / s_col[c] : 0.0;
-      if (a_on && !isfinite(a)) atomicCAS(P.ctl + C_ERR, 0, (int)POLAR_ERR_NONFINITE);
-      P.ag[c] = a;
+    if (added_split(P)) {  // mk_added completes d.v
+      for (int c = threadIdx.x; c < ld; c += blockDim.x) P.ag[c] = s_col[c];
+      return;
     }
+    if (g.nx > 0) apply_added_edges(P, red, s_col);
+    step_length(P, s_col);
+  }
+}
+
+// The added edges as a kernel of their own after the SpMM: thread item = (added-edge row,
+// column), columns consecutive over the threads, every CTA's share of d.v summed in a fixed
+// order and the last CTA finishing a.  The list is all latency (row -> offsets -> neighbours ->
+// d), so it needs many threads: with 4,096 weighted edges on 50,000 vertices (R = 64, FP64)
+// one CTA took 1,000 us of every SpMM launch (1,084 us with it, 82 without); this kernel takes
+// 20 us, and the solve went from 641 to 73 ms.
+template <typename T>
+__global__ void __launch_bounds__(kBlock) mk_added(const __grid_constant__ SolvePrm<T> P) {
+  pdl_wait();
+  pdl_launch();
+  if (!solve_live(P.ctl, P.stats, P.maxit)) return;
+  __shared__ double red[kWarps * kMaxLd];
+  __shared__ double s_col[kMaxLd];
+  const polar_graph& g = P.g;
+  const int ld = P.ld, lgld = __ffs(ld) - 1;
+  const long long nth = (long long)gridDim.x * blockDim.x;  // a multiple of ld: c is fixed
+  const int c = threadIdx.x & (ld - 1);
+  const long long items = (long long)g.nx << lgld;
+  double corr = 0.0;
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < items; q += nth) {
+    const int ix = (int)(q >> lgld);
+    const int r = __ldg(g.d_xrow + ix);
+    const int b = __ldg(g.d_xoff + ix), e = __ldg(g.d_xoff + ix + 1);
+    const double dr = (double)P.d[(size_t)r * ld + c];
+    double delta = 0.0;
+    for (int k = b; k < e; ++k) {
+      const double w = g.d_xwt ? __ldg(g.d_xwt + k) : 1.0;
+      delta += w * (dr - (double)P.d[(size_t)__ldg(g.d_xnbr + k) * ld + c]);
+    }
+    T* vp = P.v + (size_t)r * ld + c;
+    const T vold = *vp;
+    const T vnew = (T)((double)vold + delta);
+    *vp = vnew;
+    corr += dr * ((double)vnew - (double)vold);
+  }
+  red[threadIdx.x] = corr;
+  __syncthreads();
+  if (threadIdx.x < ld) {
+    double s = 0.0;
+    for (int t = threadIdx.x; t < kBlock; t += ld) s += red[t];
+    P.part[(size_t)blockIdx.x * ld + threadIdx.x] = s;
+  }
+  if (last_cta(P.ctl + C_CNTX)) {
+    reduce_partials(P.part, gridDim.x, ld, red, s_col);
+    for (int t = threadIdx.x; t < ld; t += blockDim.x) s_col[t] += P.ag[t];
+    __syncthreads();
+    step_length(P, s_col);
   }
 }
 
@@ -777,6 +846,14 @@ struct MkSolver {
     const int g4 = scaled(occ_grid(mk_dir<T, VEC>, kBlock), f, 1);
     s5 = flush_smem_for<T, E>(P);
     g5 = scaled(flush_grid<T, E>(P, s5), f, P.ld / flush_cw<T>(P.ld));
+    // added edges: one thread per (row, column) up to one CTA per SM
+    int gx = 0;
+    if (added_split(P)) {
+      const long long want = ((long long)P.g.nx * P.ld + kBlock - 1) / kBlock;
+      const int cap = scaled(sms, f, 1);
+      gx = (int)(want < cap ? want : cap);
+    }
+    const double b_added = (2.0 * s + 12.0) * P.g.nx * R;
     res.grid = g1;
     // the composed flush multiplies every history slot (zero coefficients for unused ones)
     cudaError_t e = cudaMemsetAsync(P.hist, 0, sizeof(T) * (size_t)kHist * P.nA * P.ld, st);
@@ -812,6 +889,7 @@ struct MkSolver {
     for (int k = 0; k < kHist; ++k) {
       if (P.nbh > 0) node(cs, KC_HEAVY, 0.0, [&](cudaStream_t x) { spmm_go<T, W>(1, cpl, g1, P, x); });
       node(cs, KC_SPMM, b_spmm, [&](cudaStream_t x) { spmm_go<T, W>(2, cpl, g1, P, x); });
+      if (gx > 0) node(cs, KC_ADDED, b_added, [&](cudaStream_t x) { launch_k(mk_added<T>, gx, kBlock, 0, x, P); });
       node(cs, KC_RESID, b_resid, [&](cudaStream_t x) { launch_k(mk_resid<T, VEC>, g3, kBlock, 0, x, P, k); });
       node(cs, KC_DIR, b_dir, [&](cudaStream_t x) { launch_k(mk_dir<T, VEC>, g4, kBlock, 0, x, P, k); });
     }
@@ -819,7 +897,7 @@ struct MkSolver {
     e = cudaStreamEndCapture(cs, &graph);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     if (e != cudaSuccess) return set_cuda_error("graph build", e);
-    per_block = (P.nbh > 0 ? 4 : 3) * kHist + 1;
+    per_block = (3 + (P.nbh > 0) + (gx > 0)) * kHist + 1;
     return POLAR_OK;
   }
 

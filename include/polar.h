@@ -122,7 +122,8 @@ int polar_version(void);
  * counted on class 0: 4(n+1) + 4 nnz + 2 s n R; residual, r in FP64: (16 + s) n R + s nA R;
  * direction: 24 n R (r and the direction in, the direction out; in mixed precision the
  * direction is an FP32 value plus its FP32 remainder); deferred update: (4p + M) s nA R;
- * class 7: terms of a long list of added edges). */
+ * class 7: terms of a long list of added edges; class 8: a whole solve of a small graph,
+ * with no bytes counted). */
 long long polar_launch_count(void);
 void polar_set_kernel_timing(int on);
 int polar_kernel_timing(int cls, long long* launches, double* ms, double* bytes);
@@ -174,7 +175,8 @@ int polar_msolve_finish(void* d_workspace, polar_stream_t stream, polar_msolve_i
 void polar_set_barrier_timeout_ns(uint64_t ns);
 /* Solver driver: 0 (default) one high-occupancy kernel per phase, M iterations per
  * CUDA-graph launch, host checks convergence once per launch (polar_msolve then returns
- * after the solve); 1: one persistent cooperative kernel with bounded grid barriers. */
+ * after the solve), or, for graphs whose direction fits an SM's shared memory, the whole
+ * solve in one launch of a kernel per column group (thread-block clusters); 1: one persistent cooperative kernel with bounded grid barriers. */
 int polar_set_solver_mode(int mode);
 /* Degree above which polar_msolve expects a row to be chunked for an R-column solve in
  * this precision: 8 x (lanes per row).  Heavy rows are split into chunks of at most 256

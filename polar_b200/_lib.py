@@ -140,7 +140,7 @@ def load(path=None):
     return lib
 
 
-KERNEL_CLASSES = {0: "spmm", 6: "spmm_heavy", 7: "added", 1: "resid", 2: "dir", 3: "flush", 4: "init"}
+KERNEL_CLASSES = {0: "spmm", 6: "spmm_heavy", 7: "added", 8: "cluster", 1: "resid", 2: "dir", 3: "flush", 4: "init"}
 
 
 def kernel_timing():

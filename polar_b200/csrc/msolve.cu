@@ -30,6 +30,7 @@
 #include "graph_ops.cuh"
 #include "host_util.h"
 #include "solver_core.cuh"
+#include "msolve_cl.h"
 #include "msolve_mk.h"
 #include "batch_split.h"
 
@@ -407,7 +408,8 @@ static int max_grid_for(int precision, int vec, bool weighted);
 static void solve_layout(const polar_graph* g, int precision, int R, int p, int nA, int grid, SolveLayout* L) {
   const int ld = choose_ld(precision, R);
   const size_t ts = precision == POLAR_MIXED ? 4 : 8;
-  const size_t n = g->n;
+  // the cluster solver lays the row vectors out by places, a few more than rows
+  const size_t n = g->n <= kClMaxRows ? (size_t)g->n + kClPad : (size_t)g->n;
   size_t o = 0;
   int k = 0;
   auto add = [&](size_t bytes) {
@@ -419,7 +421,8 @@ static void solve_layout(const polar_graph* g, int precision, int R, int p, int 
   add(n * ld * ts);                                // 2 v
   add((size_t)kHist * nA * ld * ts);               // 3 hist
   add((size_t)p * nA * ld * ts);                   // 4 P
-  add((size_t)p * nA * ld * ts);                   // 5 X
+  // 5 X (the cluster solver keeps it in FP64)
+  add((size_t)p * nA * ld * (g->n <= kClMaxRows ? 8 : ts));
   add((size_t)(g->nchunks > 0 ? g->nchunks : 1) * ld * 8);   // 6 chunk partials (FP64 sums)
   add((size_t)(g->nheavy > 0 ? g->nheavy : 1) * 4 * (ld > 16 ? ld / 16 : 1));  // 7 heavy counters per panel
   add((size_t)grid * ld * 8);                      // 8 CTA partials
@@ -437,6 +440,7 @@ static void solve_layout(const polar_graph* g, int precision, int R, int p, int 
   add((size_t)p * ld * kNC * 8);                   // 31 composed deferred-update coefficients
   add((size_t)kMaxHeavyCtas * ld * 8);             // 32 heavy-row d.v partials
   add(precision == POLAR_MIXED ? n * ld * 4 : 0);  // 33 direction remainder (mixed precision)
+  add(cl_graph_bytes(g, nA));                       // 34 cluster solver: row order and lists
   L->total = o;
   L->ld = ld;
   L->vec = choose_vec(precision, ld);
@@ -621,6 +625,11 @@ static void fill_prm(SolvePrm<TT>& prm, const polar_graph* g, int R, int ld, int
   prm.cmp = composed ? (double*)(ws + L.off[31]) : nullptr;
   prm.part_h = (double*)(ws + L.off[32]);
   prm.dlo = sizeof(TT) == 4 ? (float*)(ws + L.off[33]) : nullptr;
+  prm.cl.head = nullptr;
+  if (composed && g->n <= kClMaxRows) {
+    cl_graph_layout(g, nA, ws + L.off[34], &prm.cl);
+    prm.cl.X = (double*)(ws + L.off[5]);
+  }
   prm.nbh = 0;
   prm.timeout_ns = g_timeout_ns;
   // the hint path lives in the kernel-per-phase kernels only
@@ -669,14 +678,16 @@ extern "C" int polar_msolve(const polar_graph* g, int precision, const double* d
       SolvePrm<float> prm;
       fill(&prm);
       SolvePrm<float>* dp = (SolvePrm<float>*)(ws + L.off[30]);
-      if (vec == 4) rc = weighted ? mk_solve<float, 4, true, POLAR_E32>(prm, dp, st, &res) : mk_solve<float, 4, false, POLAR_E32>(prm, dp, st, &res);
+      if (cl_fits(prm)) rc = cl_solve_one(prm, st, &res);
+      else if (vec == 4) rc = weighted ? mk_solve<float, 4, true, POLAR_E32>(prm, dp, st, &res) : mk_solve<float, 4, false, POLAR_E32>(prm, dp, st, &res);
       else if (vec == 2) rc = weighted ? mk_solve<float, 2, true, POLAR_E32>(prm, dp, st, &res) : mk_solve<float, 2, false, POLAR_E32>(prm, dp, st, &res);
       else rc = weighted ? mk_solve<float, 1, true, POLAR_E32>(prm, dp, st, &res) : mk_solve<float, 1, false, POLAR_E32>(prm, dp, st, &res);
     } else {
       SolvePrm<double> prm;
       fill(&prm);
       SolvePrm<double>* dp = (SolvePrm<double>*)(ws + L.off[30]);
-      if (vec == 2) rc = weighted ? mk_solve<double, 2, true, POLAR_E64>(prm, dp, st, &res) : mk_solve<double, 2, false, POLAR_E64>(prm, dp, st, &res);
+      if (cl_fits(prm)) rc = cl_solve_one(prm, st, &res);
+      else if (vec == 2) rc = weighted ? mk_solve<double, 2, true, POLAR_E64>(prm, dp, st, &res) : mk_solve<double, 2, false, POLAR_E64>(prm, dp, st, &res);
       else rc = weighted ? mk_solve<double, 1, true, POLAR_E64>(prm, dp, st, &res) : mk_solve<double, 1, false, POLAR_E64>(prm, dp, st, &res);
     }
     if (rc != POLAR_OK) return rc;

@@ -19,6 +19,24 @@ constexpr int kMaxHeavyCtas = 1024;    // bound of the heavy-row launch (partial
 #define POLAR_E64 1  // same, FP64 iterates
 #endif
 
+// Row order of the cluster solver (msolve_cl.cu): a row's place is CTA * LS + slot.
+constexpr int kClMaxRows = 60000;  // rows up to which a workspace carries it
+constexpr int kClPad = 4096;       // places and list entries beyond the rows' own
+
+struct ClGraph {
+  int *tmp0, *tmp1;       // scratch of the sort; tmp1: rows in degree order
+  int* place;             // row -> place
+  int *srow, *sact, *sx;  // place -> row, active row in place order, added-edge row (-1: none)
+  double* sdiag;          // place -> diagonal without the shift
+  int* aorig;             // active row in place order -> the caller's
+  int2* slice;            // per slice of a CTA: first list entry, pairs of places per lane
+  int* head;              // per CTA: rows of the CTA, a warp, 8 lanes; first active row, active rows
+  unsigned short* ell;    // neighbour lists in places
+  double* ellw;           // and weights
+  double* X;              // pole iterates, FP64 in both precisions
+  int cs, LS, SL;         // CTAs, slots and table entries per CTA
+};
+
 template <typename T> struct SolvePrm {
   polar_graph g;
   int n, R, ld, p, nA;
@@ -65,6 +83,7 @@ template <typename T> struct SolvePrm {
   // data evict_first, 2: cold gathers evict_first as well.
   int hot_rows;
   int l2_mode;
+  ClGraph cl;  // cluster solver (head == nullptr: not for this workspace)
 };
 
 // Policy for a gather or store of row i of d.

@@ -25,7 +25,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .solver import max_columns, precision_code, prepare_active
+from .solver import heavy_partition, max_columns, precision_code, prepare_active
 
 __all__ = ["msolve_batch", "batch_cost"]
 
@@ -90,7 +90,8 @@ def msolve_batch(ops, Ws, taus, actives, tol, maxit=100000, track=False, *, prec
         X = torch.empty((p, nA, R), dtype=xdt, device=dev)
         h = torch.zeros((p, R), dtype=torch.float64, device=dev) if track else None
         iters = torch.zeros(R, dtype=torch.int64, device=dev)
-        gs = ops[b].struct(heavy_thresh=lib.polar_heavy_threshold(prec, R), sell_rows=lib.polar_sell_rows(prec, R))
+        thresh, chunk = heavy_partition(G, prec, R)
+        gs = ops[b].struct(heavy_thresh=thresh, sell_rows=lib.polar_sell_rows(prec, R), chunk=chunk)
         need = lib.polar_msolve_batch_workspace_bytes(gs, prec, R, p, nA)
         ws = _workspace(b, need, dev)
         q = probs[b]

@@ -238,7 +238,7 @@ class Graph:
         return self._dat_h
 
     # -- heavy-row split ---------------------------------------------------------------
-    CHUNK = 256  # neighbours per heavy-row chunk (one warp per chunk in the solver)
+    CHUNK = 256  # most neighbours per heavy-row chunk (one warp per chunk in the solver)
 
     def _split_heavy(self, thresh):
         """Default partition (threshold `thresh`) plus a cache of partitions for other
@@ -252,10 +252,10 @@ class Graph:
         self.chunk_row, self.chunk_lo, self.chunk_hi = hv["chunk_row"], hv["chunk_lo"], hv["chunk_hi"]
         self.rowblk_h, self.nrb, self.rowblk = hv["rowblk_h"], hv["nrb"], hv["rowblk"]
 
-    def _heavy_parts(self, thresh):
-        if thresh in self._heavy:
-            return self._heavy[thresh]
-        ch = self.CHUNK
+    def _heavy_parts(self, thresh, chunk=None):
+        ch = self.CHUNK if chunk is None else min(int(chunk), self.CHUNK)
+        if (thresh, ch) in self._heavy:
+            return self._heavy[thresh, ch]
         degs = np.diff(self._indptr_h.astype(np.int64))
         hrow = np.flatnonzero(degs > thresh).astype(np.int32)
         nch = -(-degs[hrow] // ch) if len(hrow) else np.zeros(0, np.int64)
@@ -276,7 +276,7 @@ class Graph:
                   hrow=_i32(hrow if len(hrow) else one, dev), hchunk_off=_i32(off, dev),
                   chunk_row=_i32(chunk_row if total else one, dev), chunk_lo=_i32(c_lo if total else one, dev),
                   chunk_hi=_i32(c_hi if total else one, dev))
-        self._heavy[thresh] = hv
+        self._heavy[thresh, ch] = hv
         return hv
 
     def Lam(self, k):
@@ -303,12 +303,13 @@ class Graph:
                                              idx=_i32(sidx if len(sidx) else np.zeros(1, np.int32), dev))
         return self._sell_cache[key]
 
-    def struct(self, extra=None, heavy_thresh=None, sell_rows=0):
+    def struct(self, extra=None, heavy_thresh=None, sell_rows=0, chunk=None):
         """ctypes polar_graph for this graph (plus an Op's added edges), with the heavy-row
-        partition for `heavy_thresh` (default: the graph's own threshold) and, when
+        partition for `heavy_thresh` (default: the graph's own threshold) in chunks of at most
+        `chunk` neighbours (default CHUNK) and, when
         sell_rows > 0 (unweighted graphs), the sliced-ELL layout of the light rows for
         warps of sell_rows rows."""
-        hv = self._heavy_parts(self.heavy_thresh if heavy_thresh is None else int(heavy_thresh))
+        hv = self._heavy_parts(self.heavy_thresh if heavy_thresh is None else int(heavy_thresh), chunk)
         s = _lib.PolarGraph()
         s.nsl = 0
         s.sell_s = 0
@@ -412,8 +413,8 @@ class Op:
         self.B.append(b)
         self._added.add(a, b, float(w))
 
-    def struct(self, heavy_thresh=None, sell_rows=0):
-        return self.G.struct(self._added, heavy_thresh=heavy_thresh, sell_rows=sell_rows)
+    def struct(self, heavy_thresh=None, sell_rows=0, chunk=None):
+        return self.G.struct(self._added, heavy_thresh=heavy_thresh, sell_rows=sell_rows, chunk=chunk)
 
     def __call__(self, x, shift=0.0):
         """Apply to an (n, R) or (n,) float64/float32 CUDA tensor; returns a new tensor."""

@@ -65,16 +65,28 @@ def _padded(prec, R):
 
 LARGE_GRAPH_ROWS = 1_000_000
 LARGE_GRAPH_HEAVY = 512
+SMALL_GRAPH_ROWS = 200_000
 
 
-def heavy_threshold(G, prec, R):
-    """Degree above which a row goes to the SpMM's warp chunks for an R-column solve: the
-    library's width rule, raised to 512 on graphs of a million rows or more, where the
-    sliced-ELL slices handle mid-degree rows with less overhead per row (measured on the
-    4M-vertex graph: R = 16 mixed 1.215 -> 1.070 ms, FP64 1.619 -> 1.481 ms, R = 128 mixed
-    6.50 -> 5.93 ms per SpMM launch, threshold 32 -> 512)."""
+def heavy_partition(G, prec, R):
+    """(threshold, chunk) of the SpMM's heavy rows for an R-column solve: rows of more
+    neighbours than the threshold go to warps in chunks of at most `chunk`.
+
+    The threshold is the library's width rule, raised to 512 on graphs of a million rows or
+    more, where the sliced-ELL slices handle mid-degree rows with less overhead per row
+    (measured on the 4M-vertex graph: R = 16 mixed 1.215 -> 1.070 ms, FP64 1.619 -> 1.481 ms,
+    R = 128 mixed 6.50 -> 5.93 ms per SpMM launch, threshold 32 -> 512).  Below that the launch
+    ends with its longest chain of gathers, not with its bytes, so long rows are cut finer the
+    fewer there are to fill the warps (FP64 / mixed, us per SpMM launch, 256-neighbour chunks at
+    the width rule -> this one: n = 50,000 R = 64 85 -> 49, n = 60,000 R = 16 39 -> 29,
+    n = 100,000 R = 128 mixed 172 -> 106, n = 317,000 R = 16 74 -> 69 and R = 128 mixed
+    326 -> 267)."""
     t = _lib.load().polar_heavy_threshold(prec, R)
-    return max(t, LARGE_GRAPH_HEAVY) if G.n >= LARGE_GRAPH_ROWS else t
+    if G.n >= LARGE_GRAPH_ROWS:
+        return max(t, LARGE_GRAPH_HEAVY), G.CHUNK
+    if G.n >= SMALL_GRAPH_ROWS:
+        return min(t, 64), 128
+    return min(t, 32), 64
 
 
 def workspace(nbytes, device):
@@ -153,8 +165,10 @@ def msolve(op, W, tau, active, tol, maxit=100000, track=False, counter=None, *, 
             lib.polar_set_spmm_lane_bytes(cfg[0])
             lib.polar_set_sell(cfg[1])
         try:
-            thresh = cfg[2] if cfg is not None else heavy_threshold(G, prec, r)
-            g = op.struct(heavy_thresh=thresh, sell_rows=lib.polar_sell_rows(prec, r))
+            thresh, chunk = heavy_partition(G, prec, r)
+            if cfg is not None:
+                thresh = cfg[2]
+            g = op.struct(heavy_thresh=thresh, sell_rows=lib.polar_sell_rows(prec, r), chunk=chunk)
             need = lib.polar_msolve_workspace_bytes(g, prec, r, p, nA)
             ws = workspace(need, dev)
             hpart = torch.zeros((p, r), dtype=torch.float64, device=dev) if track else None

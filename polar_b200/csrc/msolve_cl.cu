@@ -1051,7 +1051,7 @@ void cl_try(const SolvePrm<T>& P, int cs, ClPlan& best) {
   // reductions and scalars; gathers; the CTA's rows, dearer when their vectors come from L2;
   // the deferred update; with several CTAs their barriers and the direction's exchange.
   const double rows = (double)P.g.n / cs;
-  double c = 5000 + (0.25 + 0.02 * CG * sizeof(T)) * P.g.nnz / cs + rows * CG * (s.own ? 3.0 : 4.5) +
+  double c = 5000 + (0.25 + 0.02 * CG * sizeof(T) + (P.g.d_wts ? 0.3 : 0.0)) * P.g.nnz / cs + rows * CG * (s.own ? 3.0 : 4.5) +
              0.015 * sizeof(T) * CG * (double)P.nA * P.p / cs;
   if (cs > 1) c += 4000 + (double)P.g.n * CG * sizeof(T) / 30.0;
   s.cost = c * std::max(1.0, std::ceil((double)s.groups / most));
@@ -1137,14 +1137,17 @@ size_t cl_graph_layout(const polar_graph* g, int nA, char* base, ClGraph* C) {
   return o;
 }
 
-// The other side of the choice is the kernel-per-phase driver's iteration: 35 us of launches,
-// reductions and gather latency, then its bytes (same solves, same clocks).  The cluster
-// solver was the faster one by 1.3x to 5x at 61 of 61 shapes that fit, R = 1 to 128.
+// The other side of the choice is the kernel-per-phase driver's iteration: 45 us of launches,
+// reductions and gather latency, its vectors, gathers and deferred update (same solves, in
+// clocks).  At R = 128 the two meet near 30,000 rows (n = 29,800, 4 neighbours: 111 us an
+// iteration against 98 here; n = 28,200, 18 neighbours: 115 against 142); with fewer
+// columns the cluster solver is the faster one wherever the direction fits, by up to 2.9x.
 template <typename T>
 bool cl_fits(const SolvePrm<T>& P) {
   if (P.r32 || !P.cl.head) return false;
   const double bytes = (double)P.ld * sizeof(T);
-  return cl_plan(P).cost < 66000 + bytes * (0.016 * P.g.n + 0.0002 * P.g.nnz);
+  const double other = 85000 + bytes * (0.0076 * P.g.n + 0.00011 * P.g.nnz + 2e-5 * (4.0 * P.p + kHist) * P.nA);
+  return cl_plan(P).cost < other;
 }
 
 template <typename T>

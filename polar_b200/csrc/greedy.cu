@@ -6,6 +6,7 @@
 
 #include <cfloat>
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "host_util.h"
@@ -17,6 +18,8 @@ POLAR_D double ldx(const void* p, size_t i) {
   return (double)reinterpret_cast<const T*>(p)[i];
 }
 POLAR_D double ldv(const void* p, int f32, size_t i) { return f32 ? ldx<float>(p, i) : ldx<double>(p, i); }
+
+POLAR_HD size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // ---------------------------------------------------------------------------------------
 // W[:, c] = e_a - e_b with (a, b) = cand[sel[c]]; ia/ib = endpoint active positions.
@@ -60,8 +63,8 @@ POLAR_D bool better(double s1, long long i1, double s2, long long i2) {
   return s1 > s2 || (s1 == s2 && i1 < i2);
 }
 
-constexpr int kTopBlock = 256;
-constexpr int kTopPer = 2;  // elements per thread in the scoring and merge passes
+constexpr int kTopBlock = 256;  // candidates per CTA of the scoring pass
+constexpr int kMergeBlock = 1024;
 constexpr int kMaxB = 64;
 
 struct Cand {
@@ -98,102 +101,151 @@ POLAR_D Cand block_best(Cand c, Cand* sh) {
   return r;
 }
 
-__global__ void __launch_bounds__(kTopBlock) score_block_topb_kernel(const double* h, const double* t,
-                                                                     const double* tau, const double* om, double sigma,
-                                                                     int p, int N, const uint8_t* live, int obj, int B,
-                                                                     double* score_all, Cand* blk) {
+// Scores of one candidate per thread, kept in `score`, and each CTA's best live one.  The pass
+// is bound by its 16 p N bytes of caches: the poles are taken four at a time so that enough
+// loads are in flight, and a CTA reduces once (not B times: the B best of a million candidates
+// at p = 32, B = 16 took 199 us that way, 78 us being the caches' bytes; this pass and the
+// merge take 91 and 28).
+template <int OBJ>
+__global__ void __launch_bounds__(kTopBlock, 4) score_kernel(const double* h, const double* t, const double* tau,
+                                                          const double* om, double sigma, int p, int N,
+                                                          const uint8_t* live, double* score, Cand* best) {
   __shared__ Cand sh[33];
-  const long long base = (long long)blockIdx.x * kTopBlock * kTopPer;
-  double s[kTopPer];
-  long long idx[kTopPer];
+  const long long e = (long long)blockIdx.x * kTopBlock + threadIdx.x;
+  Cand mine{-INFINITY, LLONG_MAX};
+  if (e < N) {
+    double v;
+    if (OBJ == 1) {
+      v = log1p(t[e] + sigma * h[e]);
+    } else {
+      constexpr int U = 4;
+      double acc = 0.0;
+      for (int j0 = 0; j0 < p; j0 += U) {
+        double hj[U], tj[U];
 #pragma unroll
-  for (int k = 0; k < kTopPer; ++k) {
-    const long long e = base + (long long)k * kTopBlock + threadIdx.x;
-    idx[k] = e;
-    double v = -INFINITY;
-    if (e < N) {
-      if (obj == 1) {
-        v = log1p(t[e] + sigma * h[e]);
-      } else if (obj == 2) {
-        double acc = 0.0;
-        for (int j = 0; j < p; ++j) acc += om[j] * h[(size_t)j * N + e];
-        v = acc;
-      } else {
-        double acc = 0.0;
-        for (int j = 0; j < p; ++j) {
-          const double hj = h[(size_t)j * N + e], tj = t[(size_t)j * N + e];
-          acc += om[j] * hj / (1.0 + tj + (sigma + tau[j]) * hj);
-        }
-        v = acc;
+        for (int u = 0; u < U; ++u)
+          if (j0 + u < p) {
+            hj[u] = __ldcs(h + (size_t)(j0 + u) * N + e);
+            if (OBJ == 0) tj[u] = __ldcs(t + (size_t)(j0 + u) * N + e);
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (j0 + u < p) {
+            const int j = j0 + u;
+            if (OBJ == 2) acc += __ldg(om + j) * hj[u];
+            else acc += __ldg(om + j) * hj[u] / (1.0 + tj[u] + (sigma + __ldg(tau + j)) * hj[u]);
+          }
       }
-      if (score_all) score_all[e] = v;
-      if (!live[e]) v = -INFINITY;
-    } else {
-      idx[k] = LLONG_MAX;
+      v = acc;
     }
-    s[k] = v;
+    score[e] = v;
+    if (!live[e]) v = -INFINITY;
+    if (better(v, e, mine.s, mine.i)) mine = Cand{v, e};
   }
-  for (int b = 0; b < B; ++b) {
-    Cand mine{-INFINITY, LLONG_MAX};
-#pragma unroll
-    for (int k = 0; k < kTopPer; ++k)
-      if (idx[k] != LLONG_MAX && better(s[k], idx[k], mine.s, mine.i)) mine = Cand{s[k], idx[k]};
-    const Cand w = block_best(mine, sh);
-    if (threadIdx.x == 0) blk[(size_t)blockIdx.x * B + b] = w;
-#pragma unroll
-    for (int k = 0; k < kTopPer; ++k)
-      if (idx[k] == w.i) idx[k] = LLONG_MAX;  // taken
-  }
+  const Cand w = block_best(mine, sh);
+  if (threadIdx.x == 0) best[blockIdx.x] = w;
 }
 
-// One level of the candidate merge: each CTA keeps the B best of its 512 candidates.
-__global__ void __launch_bounds__(kTopBlock) topb_level_kernel(const Cand* in, int n_in, int B, Cand* out) {
-  __shared__ Cand sh[33];
-  double s[kTopPer];
-  long long idx[kTopPer];
-#pragma unroll
-  for (int k = 0; k < kTopPer; ++k) {
-    const long long e = (long long)blockIdx.x * kTopBlock * kTopPer + (long long)k * kTopBlock + threadIdx.x;
-    if (e < n_in) {
-      const Cand c = in[e];
-      s[k] = c.s;
-      idx[k] = c.i;
-    } else {
-      s[k] = -INFINITY;
-      idx[k] = LLONG_MAX;
-    }
-  }
-  for (int b = 0; b < B; ++b) {
-    Cand mine{-INFINITY, LLONG_MAX};
-#pragma unroll
-    for (int k = 0; k < kTopPer; ++k)
-      if (idx[k] != LLONG_MAX && better(s[k], idx[k], mine.s, mine.i)) mine = Cand{s[k], idx[k]};
-    const Cand w = block_best(mine, sh);
-    if (threadIdx.x == 0) out[(size_t)blockIdx.x * B + b] = w;
-#pragma unroll
-    for (int k = 0; k < kTopPer; ++k)
-      if (idx[k] == w.i) idx[k] = LLONG_MAX;
-  }
+// Order of the merge as integers: key of a score, larger for a better one (0: no candidate; the
+// two zeros alike), then the lower index.
+struct Ranked {
+  unsigned long long key;
+  unsigned idx;
+};
+POLAR_D unsigned long long score_key(double s) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(s + 0.0);
+  return (b >> 63) ? ~b : b | (1ull << 63);
+}
+POLAR_D double key_score(unsigned long long k) {
+  return __longlong_as_double((long long)((k >> 63) ? k ^ (1ull << 63) : ~k));
 }
 
-__global__ void __launch_bounds__(1024) merge_topb_kernel(const Cand* blk, int ncand, int B, int64_t* out_idx,
-                                                          double* out_score) {
-  __shared__ Cand sh[33];
-  extern __shared__ Cand pool[];
-  for (int i = threadIdx.x; i < ncand; i += blockDim.x) pool[i] = blk[i];
+POLAR_D Ranked warp_first(const Ranked& r) {
+  const unsigned hi = (unsigned)(r.key >> 32), lo = (unsigned)r.key;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  const bool top = hi == mh && lo == ml;
+  return Ranked{((unsigned long long)mh << 32) | ml, __reduce_min_sync(0xffffffffu, top ? r.idx : 0xffffffffu)};
+}
+
+// First of the block, in every thread, with one barrier: the warps' firsts go through `sh`
+// (two halves used in turn) and every warp reduces them.
+POLAR_D Ranked block_first(const Ranked& r, Ranked (*sh)[32], int turn) {
+  const Ranked w = warp_first(r);
+  if ((threadIdx.x & 31) == 0) sh[turn & 1][threadIdx.x >> 5] = w;
   __syncthreads();
-  for (int b = 0; b < B; ++b) {
-    Cand mine{-INFINITY, LLONG_MAX};
-    for (int i = threadIdx.x; i < ncand; i += blockDim.x)
-      if (pool[i].i != LLONG_MAX && better(pool[i].s, pool[i].i, mine.s, mine.i)) mine = pool[i];
-    const Cand w = block_best(mine, sh);
-    if (threadIdx.x == 0) {
-      out_idx[b] = w.i;
-      if (out_score) out_score[b] = w.s;
+  return warp_first(sh[turn & 1][threadIdx.x & 31]);
+}
+
+// The B best (one CTA).  An element among them lies in a scoring CTA whose own best is among
+// the B best of the CTAs' (otherwise B elements would be better than it), so those CTAs are
+// picked first and only their candidates compared.  2 B rounds of one block reduction each;
+// comparing (score, index) pairs by shuffles made a round 1.6 us.
+__global__ void __launch_bounds__(kMergeBlock) merge_topb_kernel(Cand* best, int nb, const double* score,
+                                                                 const uint8_t* live, int N, int B, int64_t* out_idx,
+                                                                 double* out_score) {
+  static_assert(kMergeBlock == 1024, "one shared entry per warp");
+  __shared__ Ranked sh[2][32];
+  __shared__ int sel[kMaxB];
+  const int tid = threadIdx.x;
+  auto before = [](const Ranked& a, const Ranked& b) { return a.key > b.key || (a.key == b.key && a.idx < b.idx); };
+  auto scan = [&]() {  // this thread's best CTA that is not taken
+    Ranked m{0, 0xffffffffu};
+    for (int i = tid; i < nb; i += kMergeBlock) {
+      const Cand c = best[i];
+      const Ranked r{c.i != LLONG_MAX ? score_key(c.s) : 0, (unsigned)c.i};
+      if (r.key && before(r, m)) m = r;
     }
-    for (int i = threadIdx.x; i < ncand; i += blockDim.x)
-      if (pool[i].i == w.i) pool[i].i = LLONG_MAX;
-    __syncthreads();
+    return m;
+  };
+  Ranked mine = scan();
+  int nsel = 0;
+  for (; nsel < B && nsel < nb; ++nsel) {
+    const Ranked w = block_first(mine, sh, nsel);
+    if (!w.key) break;
+    const int b = (int)(w.idx / kTopBlock);
+    if (tid == 0) sel[nsel] = b;
+    if (b % kMergeBlock == tid) {  // taken
+      best[b].i = LLONG_MAX;
+      mine = scan();
+    }
+  }
+  __syncthreads();
+  // candidates of this thread: position tid % kTopBlock of the CTAs tid / kTopBlock, + 4, ...
+  constexpr int W = kMergeBlock / kTopBlock;
+  constexpr int L = kMaxB / W;
+  Ranked cd[L];  // key 0: none, or taken
+#pragma unroll
+  for (int k = 0; k < L; ++k) {
+    cd[k] = Ranked{0, 0xffffffffu};
+    if (tid / kTopBlock + W * k < nsel) {
+      const long long i = (long long)sel[tid / kTopBlock + W * k] * kTopBlock + tid % kTopBlock;
+      if (i < N) {
+        const double v = live[i] ? score[i] : -INFINITY;
+        if (!isnan(v)) cd[k] = Ranked{score_key(v), (unsigned)i};
+      }
+    }
+  }
+  auto pick = [&]() {
+    Ranked m{0, 0xffffffffu};
+#pragma unroll
+    for (int k = 0; k < L; ++k)
+      if (cd[k].key && before(cd[k], m)) m = cd[k];
+    return m;
+  };
+  mine = pick();
+  for (int b = 0; b < B; ++b) {
+    const Ranked w = block_first(mine, sh, b);
+    if (tid == 0) {
+      out_idx[b] = w.key ? (int64_t)w.idx : LLONG_MAX;
+      if (out_score) out_score[b] = w.key ? key_score(w.key) : -INFINITY;
+    }
+    if (w.key && mine.idx == w.idx && mine.key == w.key) {
+#pragma unroll
+      for (int k = 0; k < L; ++k)
+        if (cd[k].idx == w.idx) cd[k].key = 0;
+      mine = pick();
+    }
   }
 }
 
@@ -235,14 +287,18 @@ __global__ void rerank_kernel(const void* U, int u_f32, int p, int nA, int ldu, 
 
 // ---------------------------------------------------------------------------------------
 // Maintenance (polar_gpu.py:242-249).
+// Row record of the maintenance: what the caches need of one (pole, active row), one sector.
+struct __align__(32) MaintRow {
+  double wx, wy, u, pad;
+};
 struct MaintTmp {
-  double *xi, *eta, *D, *nxi, *neta, *wX, *wY, *xiD, *etaD;
+  double *xi, *eta, *D, *nxi, *neta;
+  MaintRow* row;
 };
 
-POLAR_HD size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 static MaintTmp maint_tmp(void* base, int p, int nA, int q) {
-  char* b = (char*)base;
+  char* b = (char*)(((uintptr_t)base + 31) & ~uintptr_t(31));
   MaintTmp m;
   size_t o = 0;
   m.xi = (double*)(b + o); o += al256((size_t)p * q * 8);
@@ -250,15 +306,12 @@ static MaintTmp maint_tmp(void* base, int p, int nA, int q) {
   m.D = (double*)(b + o); o += al256((size_t)p * 8);
   m.nxi = (double*)(b + o); o += al256((size_t)p * 8);
   m.neta = (double*)(b + o); o += al256((size_t)p * 8);
-  m.wX = (double*)(b + o); o += al256((size_t)p * nA * 8);
-  m.wY = (double*)(b + o); o += al256((size_t)p * nA * 8);
-  m.xiD = (double*)(b + o); o += al256((size_t)p * q * 8);
-  m.etaD = (double*)(b + o); o += al256((size_t)p * q * 8);
+  m.row = (MaintRow*)(b + o);
   return m;
 }
 
 static size_t maint_tmp_bytes(int p, int nA, int q) {
-  return al256((size_t)p * q * 8) * 4 + al256((size_t)p * 8) * 3 + al256((size_t)p * nA * 8) * 2;
+  return al256((size_t)p * q * 8) * 2 + al256((size_t)p * 8) * 3 + al256((size_t)p * nA * sizeof(MaintRow)) + 32;
 }
 
 // one CTA per pole
@@ -290,96 +343,114 @@ __global__ void maint_setup_kernel(const void* X, int ldx, const void* Y, int ld
     }
     m.nxi[j] = t1;
     m.neta[j] = t2;
-    s1[0] = 1.0 + ldv(U, u_f32, ((size_t)j * nA + a) * ldu + uc) - ldv(U, u_f32, ((size_t)j * nA + b) * ldu + uc);
-    m.D[j] = s1[0];
-  }
-  __syncthreads();
-  const double D = s1[0];
-  for (int c = threadIdx.x; c < q; c += blockDim.x) {
-    m.xiD[(size_t)j * q + c] = m.xi[(size_t)j * q + c] / D;
-    m.etaD[(size_t)j * q + c] = m.eta[(size_t)j * q + c] / D;
+    m.D[j] = 1.0 + ldv(U, u_f32, ((size_t)j * nA + a) * ldu + uc) - ldv(U, u_f32, ((size_t)j * nA + b) * ldu + uc);
   }
 }
 
-// One 16-lane group per (pole, active row): w = row . dir (before the update), then
-// X_row -= u xi/D, Y_row += u eta/D.  Lanes own VEC consecutive columns (vector loads).
-template <typename T, int VEC>
-__global__ void maint_rows_kernel(T* X, int ldx, T* Y, int ldy, int p, int nA, int q, const void* U, int u_f32,
-                                  int ldu, const int32_t* win, MaintTmp m) {
-  const int lanes = 16;
-  const long long gidx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / lanes;
-  const int lg = threadIdx.x & (lanes - 1);
-  const unsigned mask = 0xffffu << (threadIdx.x & 16);
-  if (gidx >= (long long)p * nA) return;
-  const int j = (int)(gidx / nA), a = (int)(gidx % nA);
+// w = row . dir (before the update), then X_row -= u xi / D, Y_row += u eta / D, for the rows of
+// one pole (blockIdx.y): 8 lanes per row, each with NT x VEC of its columns, whose xi and eta
+// stay in registers over the CTA's rows (reading them again for every row was 2 KB from L1 for
+// the row's own 512 bytes: 2,210 us at 24 x 226,000 rows, q = 64 mixed; 1,050 us now, the
+// bytes of X and Y being 850).
+constexpr int kMaintBlock = 256;
+constexpr int kMaintRows = 512;  // rows per CTA
+
+template <typename T, int VEC, int NT>
+__global__ void __launch_bounds__(kMaintBlock, NT <= 2 ? 3 : 1) maint_rows_kernel(T* X, int ldx, T* Y, int ldy, int nA, int q, int c0,
+                                                                 int c1, const void* U, int u_f32, int ldu,
+                                                                 const int32_t* win, MaintTmp m) {
+  // columns [c0, c1) of q (a wide bank goes in several launches, whose dots add up)
+  constexpr int LPR = 8;
+  const int j = blockIdx.y, lg = threadIdx.x & (LPR - 1);
   const int uc = win[0];
-  const double u = ldv(U, u_f32, ((size_t)j * nA + a) * ldu + uc);
-  T* xr = X + ((size_t)j * nA + a) * ldx;
-  T* yr = Y + ((size_t)j * nA + a) * ldy;
-  const double* xi = m.xi + (size_t)j * q;
-  const double* eta = m.eta + (size_t)j * q;
-  const double* xiD = m.xiD + (size_t)j * q;
-  const double* etaD = m.etaD + (size_t)j * q;
-  double wx = 0.0, wy = 0.0;
-  for (int c = lg * VEC; c < q; c += lanes * VEC) {
-    T xv[VEC], yv[VEC];
-    vload<T, VEC>(xv, xr + c);
-    vload<T, VEC>(yv, yr + c);
+  const double D = m.D[j], rD = 1.0 / D;
+  double xi[NT][VEC], eta[NT][VEC];
+#pragma unroll
+  for (int k = 0; k < NT; ++k)
 #pragma unroll
     for (int v = 0; v < VEC; ++v) {
-      const double x = (double)xv[v], y = (double)yv[v];
-      wx = fma(x, __ldg(xi + c + v), wx);
-      wy = fma(y, __ldg(eta + c + v), wy);
-      xv[v] = (T)fma(-u, __ldg(xiD + c + v), x);
-      yv[v] = (T)fma(u, __ldg(etaD + c + v), y);
+      const int c = c0 + (k * LPR + lg) * VEC + v;
+      xi[k][v] = c < c1 ? m.xi[(size_t)j * q + c] : 0.0;
+      eta[k][v] = c < c1 ? m.eta[(size_t)j * q + c] : 0.0;
     }
-    vstore<T, VEC>(xr + c, xv);
-    vstore<T, VEC>(yr + c, yv);
-  }
-  for (int o = 8; o > 0; o >>= 1) {
-    wx += __shfl_xor_sync(mask, wx, o);
-    wy += __shfl_xor_sync(mask, wy, o);
-  }
-  if (lg == 0) {
-    m.wX[gidx] = wx;
-    m.wY[gidx] = wy;
+  const int a1 = min(nA, (int)(blockIdx.x + 1) * kMaintRows);
+  for (int a0 = blockIdx.x * kMaintRows; a0 < a1; a0 += kMaintBlock / LPR) {
+    const int a = a0 + threadIdx.x / LPR;
+    const bool ok = a < a1;
+    T xv[NT][VEC], yv[NT][VEC];
+    double u = 0.0, wx = 0.0, wy = 0.0;
+    T* const xr = X + ((size_t)j * nA + a) * ldx;
+    T* const yr = Y + ((size_t)j * nA + a) * ldy;
+    if (ok) {
+#pragma unroll
+      for (int k = 0; k < NT; ++k) {
+        const int c = c0 + (k * LPR + lg) * VEC;
+        if (c < c1) {
+          vload<T, VEC>(xv[k], xr + c);
+          vload<T, VEC>(yv[k], yr + c);
+        }
+      }
+      u = ldv(U, u_f32, ((size_t)j * nA + a) * ldu + uc);
+      const double q0 = u * rD;
+      const double ud = fma(fma(-q0, D, u), rD, q0);  // u / D
+#pragma unroll
+      for (int k = 0; k < NT; ++k) {
+        const int c = c0 + (k * LPR + lg) * VEC;
+        if (c < c1) {
+#pragma unroll
+          for (int v = 0; v < VEC; ++v) {
+            const double x = (double)xv[k][v], y = (double)yv[k][v];
+            wx = fma(x, xi[k][v], wx);
+            wy = fma(y, eta[k][v], wy);
+            xv[k][v] = (T)fma(-ud, xi[k][v], x);
+            yv[k][v] = (T)fma(ud, eta[k][v], y);
+          }
+          vstore<T, VEC>(xr + c, xv[k]);
+          vstore<T, VEC>(yr + c, yv[k]);
+        }
+      }
+    }
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) {
+      wx += __shfl_xor_sync(0xffffffffu, wx, o);
+      wy += __shfl_xor_sync(0xffffffffu, wy, o);
+    }
+    if (ok && lg == 0) {
+      MaintRow& r = m.row[(size_t)j * nA + a];
+      if (c0 > 0) {
+        wx += r.wx;
+        wy += r.wy;
+      }
+      r = MaintRow{wx, wy, u, 0.0};
+    }
   }
 }
 
-__global__ void maint_cache_kernel(int p, int nA, int N, const void* U, int u_f32, int ldu, const int32_t* win,
-                                   const int32_t* es, MaintTmp m, double* h, double* t) {
+// Cache change of item (pole j, candidate e): its two row records are one sector each.
+POLAR_D void maint_change(const MaintTmp& m, const int32_t* es, int nA, int j, int e, double& dh, double& dt) {
+  const MaintRow ra = m.row[(size_t)j * nA + es[2 * (size_t)e]], rb = m.row[(size_t)j * nA + es[2 * (size_t)e + 1]];
+  const double cc = (ra.u - rb.u) / m.D[j];
+  dh = cc * cc * m.nxi[j] - 2.0 * cc * (ra.wx - rb.wx);
+  dt = cc * cc * m.neta[j] + 2.0 * cc * (ra.wy - rb.wy);
+}
+
+__global__ void maint_cache_kernel(int p, int nA, int N, const int32_t* es, MaintTmp m, double* h, double* t) {
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (long long)p * N) return;
   const int j = (int)(g / N), e = (int)(g % N);
-  const int uc = win[0];
-  const int32_t* ea = es;
-  const int32_t* eb = es + 1;
-  const int a = ea[2 * e], b = eb[2 * e];
-  const double cc = (ldv(U, u_f32, ((size_t)j * nA + a) * ldu + uc) - ldv(U, u_f32, ((size_t)j * nA + b) * ldu + uc)) /
-                    m.D[j];
-  const double dx = m.wX[(size_t)j * nA + a] - m.wX[(size_t)j * nA + b];
-  const double dy = m.wY[(size_t)j * nA + a] - m.wY[(size_t)j * nA + b];
-  const size_t o = (size_t)j * N + e;
-  h[o] = fmax(0.0, h[o] - 2.0 * cc * dx + cc * cc * m.nxi[j]);
-  t[o] = fmax(0.0, t[o] + 2.0 * cc * dy + cc * cc * m.neta[j]);
+  double dh, dt;
+  maint_change(m, es, nA, j, e, dh, dt);
+  h[g] = fmax(0.0, h[g] + dh);
+  t[g] = fmax(0.0, t[g] + dt);
 }
 
 // Column-split form (the sketch columns spread over several ranks): this rank's share of
 // the cache change, summed over the ranks before cache_apply_kernel clamps it in.
-__global__ void maint_delta_kernel(int p, int nA, int N, const void* U, int u_f32, int ldu, const int32_t* win,
-                                   const int32_t* es, MaintTmp m, double* dh, double* dt) {
+__global__ void maint_delta_kernel(int p, int nA, int N, const int32_t* es, MaintTmp m, double* dh, double* dt) {
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (long long)p * N) return;
   const int j = (int)(g / N), e = (int)(g % N);
-  const int uc = win[0];
-  const int a = es[2 * e], b = es[2 * e + 1];
-  const double cc = (ldv(U, u_f32, ((size_t)j * nA + a) * ldu + uc) - ldv(U, u_f32, ((size_t)j * nA + b) * ldu + uc)) /
-                    m.D[j];
-  const double dx = m.wX[(size_t)j * nA + a] - m.wX[(size_t)j * nA + b];
-  const double dy = m.wY[(size_t)j * nA + a] - m.wY[(size_t)j * nA + b];
-  const size_t o = (size_t)j * N + e;
-  dh[o] = cc * cc * m.nxi[j] - 2.0 * cc * dx;
-  dt[o] = cc * cc * m.neta[j] + 2.0 * cc * dy;
+  maint_change(m, es, nA, j, e, dh[g], dt[g]);
 }
 
 __global__ void cache_apply_kernel(double* h, const double* dh, double* t, const double* dt, long long count) {
@@ -453,9 +524,9 @@ extern "C" int polar_pair_norms(const void* d_X, int x_f32, int p, int nA, int l
 }
 
 extern "C" size_t polar_topb_tmp_bytes(int N, int B) {
-  const long long per = (long long)kTopBlock * kTopPer;
-  const long long nb = (N + per - 1) / per;
-  return 2 * (size_t)(nb > 0 ? nb : 1) * (B > 0 ? B : 1) * sizeof(Cand) + 256;
+  (void)B;
+  const size_t n = N > 0 ? N : 1;
+  return al256(n * sizeof(double)) + (n + kTopBlock - 1) / kTopBlock * sizeof(Cand) + 256;
 }
 
 extern "C" int polar_score_topb(const double* d_h, const double* d_t, const double* d_tau, const double* d_om,
@@ -466,32 +537,15 @@ extern "C" int polar_score_topb(const double* d_h, const double* d_t, const doub
     return set_error(POLAR_ERR_BAD_ARG, "bad arguments");
   if (B < 1 || B > kMaxB || B > N) return set_error(POLAR_ERR_BAD_ARG, "B out of range");
   if (obj < 0 || obj > 2) return set_error(POLAR_ERR_BAD_ARG, "obj must be 0, 1 or 2");
-  const long long per = (long long)kTopBlock * kTopPer;
-  const int nb = (int)((N + per - 1) / per);
+  const int nb = (int)(((long long)N + kTopBlock - 1) / kTopBlock);
   cudaStream_t st = (cudaStream_t)stream;
-  score_block_topb_kernel<<<nb, kTopBlock, 0, st>>>(d_h, d_t, d_tau, d_om, sigma, p, N, d_live, obj, B, d_score_all,
-                                                    (Cand*)d_tmp);
-  int rc = check_launch("score_block_topb");
+  double* score = d_score_all ? d_score_all : (double*)d_tmp;
+  Cand* best = (Cand*)((char*)d_tmp + al256((size_t)N * sizeof(double)));
+  auto* k = obj == 1 ? score_kernel<1> : obj == 2 ? score_kernel<2> : score_kernel<0>;
+  k<<<nb, kTopBlock, 0, st>>>(d_h, d_t, d_tau, d_om, sigma, p, N, d_live, score, best);
+  const int rc = check_launch("score");
   if (rc) return rc;
-  // merge levels until one CTA can take the rest
-  const long long per_lvl = (long long)kTopBlock * kTopPer;
-  Cand* a = (Cand*)d_tmp;
-  Cand* b2 = a + (size_t)nb * B;
-  long long ncand = (long long)nb * B;
-  while (ncand > 4096) {
-    const int nb2 = (int)((ncand + per_lvl - 1) / per_lvl);
-    topb_level_kernel<<<nb2, kTopBlock, 0, st>>>(a, (int)ncand, B, b2);
-    rc = check_launch("topb_level");
-    if (rc) return rc;
-    Cand* t = a;
-    a = b2;
-    b2 = t;
-    ncand = (long long)nb2 * B;
-  }
-  const size_t smem = (size_t)ncand * sizeof(Cand);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(merge_topb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  merge_topb_kernel<<<1, 1024, smem, st>>>(a, (int)ncand, B, d_out_idx, d_out_score);
+  merge_topb_kernel<<<1, kMergeBlock, 0, st>>>(best, nb, score, d_live, N, B, d_out_idx, d_out_score);
   return check_launch("merge_topb");
 }
 
@@ -531,32 +585,43 @@ static int maintain(void* d_X, int ldx, void* d_Y, int ldy, int xy_f32, int p, i
   maint_setup_kernel<<<p, 128, 0, st>>>(d_X, ldx, d_Y, ldy, xy_f32, p, nA, q, d_U, u_f32, ldu, d_win, d_G, m);
   int rc = check_launch("maint_setup");
   if (rc) return rc;
-  const long long thr = (long long)p * nA * 16;
-  const int blocks = (int)((thr + 255) / 256);
   const uintptr_t al = (uintptr_t)d_X | (uintptr_t)d_Y;
+  const dim3 grid((nA + kMaintRows - 1) / kMaintRows, p);
+  auto rows = [&](auto* x, auto* y, auto vec) {
+    using T = std::remove_pointer_t<decltype(x)>;
+    constexpr int V = decltype(vec)::value;
+    for (int c0 = 0; c0 < q; c0 += 8 * 8 * V) {
+      const int c1 = q - c0 < 8 * 8 * V ? q : c0 + 8 * 8 * V;
+      const int trips = (c1 - c0 + 8 * V - 1) / (8 * V);
+      auto go = [&](auto nt) {
+        maint_rows_kernel<T, V, decltype(nt)::value><<<grid, kMaintBlock, 0, st>>>(x, ldx, y, ldy, nA, q, c0, c1, d_U,
+                                                                                   u_f32, ldu, d_win, m);
+      };
+      if (trips <= 1) go(std::integral_constant<int, 1>{});
+      else if (trips <= 2) go(std::integral_constant<int, 2>{});
+      else if (trips <= 4) go(std::integral_constant<int, 4>{});
+      else go(std::integral_constant<int, 8>{});
+    }
+  };
   if (xy_f32) {
     if (q % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 && al % 16 == 0)
-      maint_rows_kernel<float, 4><<<blocks, 256, 0, st>>>((float*)d_X, ldx, (float*)d_Y, ldy, p, nA, q, d_U, u_f32,
-                                                          ldu, d_win, m);
+      rows((float*)d_X, (float*)d_Y, std::integral_constant<int, 4>{});
     else
-      maint_rows_kernel<float, 1><<<blocks, 256, 0, st>>>((float*)d_X, ldx, (float*)d_Y, ldy, p, nA, q, d_U, u_f32,
-                                                          ldu, d_win, m);
+      rows((float*)d_X, (float*)d_Y, std::integral_constant<int, 1>{});
   } else {
     if (q % 2 == 0 && ldx % 2 == 0 && ldy % 2 == 0 && al % 16 == 0)
-      maint_rows_kernel<double, 2><<<blocks, 256, 0, st>>>((double*)d_X, ldx, (double*)d_Y, ldy, p, nA, q, d_U,
-                                                           u_f32, ldu, d_win, m);
+      rows((double*)d_X, (double*)d_Y, std::integral_constant<int, 2>{});
     else
-      maint_rows_kernel<double, 1><<<blocks, 256, 0, st>>>((double*)d_X, ldx, (double*)d_Y, ldy, p, nA, q, d_U,
-                                                           u_f32, ldu, d_win, m);
+      rows((double*)d_X, (double*)d_Y, std::integral_constant<int, 1>{});
   }
   rc = check_launch("maint_rows");
   if (rc) return rc;
   if (N > 0) {
     const long long t2 = (long long)p * N;
     if (delta)
-      maint_delta_kernel<<<(int)((t2 + 255) / 256), 256, 0, st>>>(p, nA, N, d_U, u_f32, ldu, d_win, d_es, m, d_h, d_t);
+      maint_delta_kernel<<<(int)((t2 + 255) / 256), 256, 0, st>>>(p, nA, N, d_es, m, d_h, d_t);
     else
-      maint_cache_kernel<<<(int)((t2 + 255) / 256), 256, 0, st>>>(p, nA, N, d_U, u_f32, ldu, d_win, d_es, m, d_h, d_t);
+      maint_cache_kernel<<<(int)((t2 + 255) / 256), 256, 0, st>>>(p, nA, N, d_es, m, d_h, d_t);
     rc = check_launch(delta ? "maint_delta" : "maint_cache");
   }
   return rc;

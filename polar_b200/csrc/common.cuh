@@ -32,8 +32,66 @@ struct VecWidth {
   static constexpr int value = (V * (int)sizeof(T) <= 16) ? V : 16 / (int)sizeof(T);
 };
 
-template <typename T, int V>
+// 32 bytes through one 256-bit access (sm_100).  A lane that owns 32 consecutive bytes and reads
+// them as two 16-byte accesses makes each of the warp's accesses touch every line of the rows
+// it reads, so L1 looks every line up twice; one 256-bit access looks it up once.  The SpMM
+// gathers of 512-byte rows were bound by that (82 % of the L1 throughput, L2 at 24 %, half of
+// the look-ups hits on the first access's lines).  Global memory, 32-byte aligned only: the
+// W32 parameter below says that the caller's rows are.
+POLAR_D void ld32(float* o, const float* p) {
+  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
+               : "l"(p));
+}
+POLAR_D void ld32(double* o, const double* p) {
+  asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+               : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3]) : "l"(p));
+}
+POLAR_D void ld32_hint(float* o, const float* p, uint64_t pol) {
+  asm volatile("ld.global.L2::cache_hint.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;"
+               : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
+               : "l"(p), "l"(pol));
+}
+POLAR_D void ld32_hint(double* o, const double* p, uint64_t pol) {
+  asm volatile("ld.global.L2::cache_hint.v4.f64 {%0,%1,%2,%3}, [%4], %5;"
+               : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3]) : "l"(p), "l"(pol));
+}
+POLAR_D void st32(float* p, const float* i) {
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"l"(p), "f"(i[0]), "f"(i[1]), "f"(i[2]), "f"(i[3]), "f"(i[4]), "f"(i[5]), "f"(i[6]), "f"(i[7]) : "memory");
+}
+POLAR_D void st32(double* p, const double* i) {
+  asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(p), "d"(i[0]), "d"(i[1]), "d"(i[2]), "d"(i[3]) : "memory");
+}
+POLAR_D void st32_cs(float* p, const float* i) {
+  asm volatile("st.global.cs.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"l"(p), "f"(i[0]), "f"(i[1]), "f"(i[2]), "f"(i[3]), "f"(i[4]), "f"(i[5]), "f"(i[6]), "f"(i[7]) : "memory");
+}
+POLAR_D void st32_cs(double* p, const double* i) {
+  asm volatile("st.global.cs.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(p), "d"(i[0]), "d"(i[1]), "d"(i[2]), "d"(i[3]) : "memory");
+}
+POLAR_D void st32_hint(float* p, const float* i, uint64_t pol) {
+  asm volatile("st.global.L2::cache_hint.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8}, %9;"
+               ::"l"(p), "f"(i[0]), "f"(i[1]), "f"(i[2]), "f"(i[3]), "f"(i[4]), "f"(i[5]), "f"(i[6]), "f"(i[7]), "l"(pol)
+               : "memory");
+}
+POLAR_D void st32_hint(double* p, const double* i, uint64_t pol) {
+  asm volatile("st.global.L2::cache_hint.v4.f64 [%0], {%1,%2,%3,%4}, %5;"
+               ::"l"(p), "d"(i[0]), "d"(i[1]), "d"(i[2]), "d"(i[3]), "l"(pol) : "memory");
+}
+// Whole 256-bit accesses of V elements: taken when the caller vouches for the alignment.
+template <typename T, int V, bool W32>
+POLAR_HD constexpr bool takes32() {
+  return W32 && (V * (int)sizeof(T)) % 32 == 0;
+}
+
+template <typename T, int V, bool W32 = false>
 POLAR_D void vload(T (&out)[V], const T* p) {
+  if constexpr (takes32<T, V, W32>()) {
+#pragma unroll
+    for (int c = 0; c < V; c += 32 / (int)sizeof(T)) ld32(out + c, p + c);
+    return;
+  }
   constexpr int VW = VecWidth<T, V>::value;
 #pragma unroll
   for (int c = 0; c < V / VW; ++c) {
@@ -57,8 +115,13 @@ POLAR_D void vload_cg(T (&out)[V], const T* p) {
   }
 }
 
-template <typename T, int V>
+template <typename T, int V, bool W32 = false>
 POLAR_D void vstore(T* p, const T (&in)[V]) {
+  if constexpr (takes32<T, V, W32>()) {
+#pragma unroll
+    for (int c = 0; c < V; c += 32 / (int)sizeof(T)) st32(p + c, in + c);
+    return;
+  }
   constexpr int VW = VecWidth<T, V>::value;
 #pragma unroll
   for (int c = 0; c < V / VW; ++c) {
@@ -70,8 +133,13 @@ POLAR_D void vstore(T* p, const T (&in)[V]) {
 }
 
 // Evict-first (streaming) store, for data that is not read again soon.
-template <typename T, int V>
+template <typename T, int V, bool W32 = false>
 POLAR_D void vstore_cs(T* p, const T (&in)[V]) {
+  if constexpr (takes32<T, V, W32>()) {
+#pragma unroll
+    for (int c = 0; c < V; c += 32 / (int)sizeof(T)) st32_cs(p + c, in + c);
+    return;
+  }
   constexpr int VW = VecWidth<T, V>::value;
 #pragma unroll
   for (int c = 0; c < V / VW; ++c) {
@@ -137,8 +205,13 @@ POLAR_D void st_hint(void* p, const double& v, uint64_t pol) {
   asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(p), "d"(v), "l"(pol) : "memory");
 }
 
-template <typename T, int V>
+template <typename T, int V, bool W32 = false>
 POLAR_D void vload_hint(T (&out)[V], const T* p, uint64_t pol) {
+  if constexpr (takes32<T, V, W32>()) {
+#pragma unroll
+    for (int c = 0; c < V; c += 32 / (int)sizeof(T)) ld32_hint(out + c, p + c, pol);
+    return;
+  }
   constexpr int VW = VecWidth<T, V>::value;
 #pragma unroll
   for (int c = 0; c < V / VW; ++c) {
@@ -149,8 +222,13 @@ POLAR_D void vload_hint(T (&out)[V], const T* p, uint64_t pol) {
   }
 }
 
-template <typename T, int V>
+template <typename T, int V, bool W32 = false>
 POLAR_D void vstore_hint(T* p, const T (&in)[V], uint64_t pol) {
+  if constexpr (takes32<T, V, W32>()) {
+#pragma unroll
+    for (int c = 0; c < V; c += 32 / (int)sizeof(T)) st32_hint(p + c, in + c, pol);
+    return;
+  }
   constexpr int VW = VecWidth<T, V>::value;
 #pragma unroll
   for (int c = 0; c < V / VW; ++c) {

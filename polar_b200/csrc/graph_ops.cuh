@@ -51,7 +51,7 @@ POLAR_D RowGroup make_row_group(int ld) {
 // cooperatively and broadcast them by shuffles; narrower groups read the next 4 indices
 // directly (the same addresses for the group's lanes, served by L1) so 4 gathers are in
 // flight per lane.
-template <typename T, int VEC, bool WEIGHTED, typename AA = typename AccOf<T>::type>
+template <typename T, int VEC, bool WEIGHTED, typename AA = typename AccOf<T>::type, bool W32 = false>
 POLAR_D void gather_rows(const polar_graph& g, const RowGroup& rg, int lo, int hi, const T* X,
                          int ld, AA (&acc)[VEC], bool on = true) {
   using A = AA;
@@ -68,7 +68,7 @@ POLAR_D void gather_rows(const polar_graph& g, const RowGroup& rg, int lo, int h
       }
       T xv[4][VEC];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) vload<T, VEC>(xv[u], X + (size_t)jj[u] * ld + rg.col);
+      for (int u = 0; u < 4; ++u) vload<T, VEC, W32>(xv[u], X + (size_t)jj[u] * ld + rg.col);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -78,7 +78,7 @@ POLAR_D void gather_rows(const polar_graph& g, const RowGroup& rg, int lo, int h
       const int jj = __ldg(g.d_indices + k);
       const A ww = WEIGHTED ? (A)__ldg(g.d_wts + k) : A(1);
       T xv[VEC];
-      vload<T, VEC>(xv, X + (size_t)jj * ld + rg.col);
+      vload<T, VEC, W32>(xv, X + (size_t)jj * ld + rg.col);
 #pragma unroll
       for (int v = 0; v < VEC; ++v) acc[v] = WEIGHTED ? fma(ww, (A)xv[v], acc[v]) : acc[v] + (A)xv[v];
     }
@@ -105,7 +105,7 @@ POLAR_D void gather_rows(const polar_graph& g, const RowGroup& rg, int lo, int h
       if (on) {
         T xv[4][VEC];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) vload<T, VEC>(xv[u], X + (size_t)jj[u] * ld + rg.col);
+        for (int u = 0; u < 4; ++u) vload<T, VEC, W32>(xv[u], X + (size_t)jj[u] * ld + rg.col);
 #pragma unroll
         for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -117,7 +117,7 @@ POLAR_D void gather_rows(const polar_graph& g, const RowGroup& rg, int lo, int h
       const A ww = WEIGHTED ? __shfl_sync(rg.mask, w, t, rg.G) : A(1);
       if (on) {
         T xv[VEC];
-        vload<T, VEC>(xv, X + (size_t)jj * ld + rg.col);
+        vload<T, VEC, W32>(xv, X + (size_t)jj * ld + rg.col);
 #pragma unroll
         for (int v = 0; v < VEC; ++v) acc[v] = WEIGHTED ? fma(ww, (A)xv[v], acc[v]) : acc[v] + (A)xv[v];
       }
@@ -154,7 +154,7 @@ POLAR_D double added_terms(const polar_graph& g, const RowGroup& rg, int i, cons
 
 // Finishes row i from its own entries xi (already loaded): y = (diag + shift) x_i - acc.
 // ADD = false leaves out the added edges (the caller applies them afterwards).
-template <typename T, int VEC, bool ADD = true, typename AA = typename AccOf<T>::type>
+template <typename T, int VEC, bool ADD = true, typename AA = typename AccOf<T>::type, bool W32 = false>
 POLAR_D void finish_row_pre(const polar_graph& g, const RowGroup& rg, int i, int deg, double shift, const T* X,
                             int ld, AA (&acc)[VEC], T* Y, int ldy, const T (&xi)[VEC],
                             T (&yi)[VEC], bool store = true) {
@@ -169,11 +169,11 @@ POLAR_D void finish_row_pre(const polar_graph& g, const RowGroup& rg, int i, int
   const double dg = (g.d_diag ? __ldg(g.d_diag + i) : (double)deg + g.sigma) + wadd + shift;
 #pragma unroll
   for (int v = 0; v < VEC; ++v) yi[v] = (T)fma((A)dg, (A)xi[v], -acc[v]);
-  vstore<T, VEC>(Y + (size_t)i * ldy + rg.col, yi);
+  vstore<T, VEC, W32>(Y + (size_t)i * ldy + rg.col, yi);
 }
 
 // Finishes row i: y = (diag + shift) x_i - acc.  Returns x_i in xi (for d^T v).
-template <typename T, int VEC, bool ADD = true, typename AA = typename AccOf<T>::type>
+template <typename T, int VEC, bool ADD = true, typename AA = typename AccOf<T>::type, bool W32 = false>
 POLAR_D void finish_row(const polar_graph& g, const RowGroup& rg, int i, int deg, double shift,
                         const T* X, int ld, AA (&acc)[VEC], T* Y,
                         int ldy, T (&xi)[VEC], T (&yi)[VEC], bool store = true) {
@@ -186,10 +186,10 @@ POLAR_D void finish_row(const polar_graph& g, const RowGroup& rg, int i, int deg
   double wadd = 0.0;
   if constexpr (ADD) wadd = added_terms<T, VEC, AA>(g, rg, i, X, ld, acc);
   const double dg = (g.d_diag ? __ldg(g.d_diag + i) : (double)deg + g.sigma) + wadd + shift;
-  vload<T, VEC>(xi, X + (size_t)i * ld + rg.col);
+  vload<T, VEC, W32>(xi, X + (size_t)i * ld + rg.col);
 #pragma unroll
   for (int v = 0; v < VEC; ++v) yi[v] = (T)fma((A)dg, (A)xi[v], -acc[v]);
-  if (store) vstore<T, VEC>(Y + (size_t)i * ldy + rg.col, yi);
+  if (store) vstore<T, VEC, W32>(Y + (size_t)i * ldy + rg.col, yi);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -401,7 +401,9 @@ static int choose_ld(int precision, int R) {
 
 static int max_ld(int precision) { return precision == POLAR_MIXED ? 128 : 64; }
 
-static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
+constexpr size_t kWsAlign = 256;
+static size_t align256(size_t x) { return (x + kWsAlign - 1) & ~(kWsAlign - 1); }
+static char* ws_base(void* ws) { return (char*)align256((size_t)ws); }
 
 static int max_grid_for(int precision, int vec, bool weighted);
 
@@ -441,7 +443,7 @@ static void solve_layout(const polar_graph* g, int precision, int R, int p, int 
   add((size_t)kMaxHeavyCtas * ld * 8);             // 32 heavy-row d.v partials
   add(precision == POLAR_MIXED ? n * ld * 4 : 0);  // 33 direction remainder (mixed precision)
   add(cl_graph_bytes(g, nA));                       // 34 cluster solver: row order and lists
-  L->total = o;
+  L->total = o + kWsAlign;  // the regions start at the first aligned byte of the workspace
   L->ld = ld;
   L->vec = choose_vec(precision, ld);
 }
@@ -658,7 +660,7 @@ extern "C" int polar_msolve(const polar_graph* g, int precision, const double* d
   solve_layout(g, precision, R, p, nA, grid, &L);
   if (workspace_bytes < L.total) return set_error(POLAR_ERR_WORKSPACE, "workspace too small");
   cudaStream_t st = (cudaStream_t)stream;
-  char* ws = (char*)d_workspace;
+  char* ws = ws_base(d_workspace);
   // zero the small control/state regions the kernel expects cleared
   cudaError_t e;
   e = cudaMemsetAsync(ws + L.off[27], 0, 64, st);
@@ -812,7 +814,7 @@ static int batch_graph_run(const polar_msolve_problem* probs, int nprob, int ld,
   const int full = mk_grid_max<T, VEC, W, E>();
   for (int b = 0; b < nprob; ++b) {
     const polar_msolve_problem& q = probs[b];
-    char* ws = (char*)q.d_workspace;
+    char* ws = ws_base(q.d_workspace);
     cudaError_t e = cudaMemsetAsync(ws + L[b].off[27], 0, 64, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(ws + L[b].off[28], 0, 64, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(ws + L[b].off[7], 0, L[b].off[8] - L[b].off[7], st);
@@ -921,7 +923,7 @@ extern "C" int polar_msolve_batch(const polar_msolve_problem* probs, int nprob, 
   const int grid = B.cta_off[nprob];
   for (int b = 0; b < nprob; ++b) {
     const polar_msolve_problem& q = probs[b];
-    char* ws = (char*)q.d_workspace;
+    char* ws = ws_base(q.d_workspace);
     cudaError_t e = cudaMemsetAsync(ws + L[b].off[27], 0, 64, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(ws + L[b].off[28], 0, 64, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(ws + L[b].off[7], 0, L[b].off[8] - L[b].off[7], st);
@@ -952,7 +954,7 @@ extern "C" int polar_msolve_batch(const polar_msolve_problem* probs, int nprob, 
   }
   if (rc != POLAR_OK) return rc;
   for (int b = 0; b < nprob; ++b) {
-    char* ws = (char*)probs[b].d_workspace;
+    char* ws = ws_base(probs[b].d_workspace);
     remember_solve(probs[b].d_workspace, (int*)(ws + L[b].off[27]), (long long*)(ws + L[b].off[28]), ld, ctas[b], kBlock);
   }
   return POLAR_OK;

@@ -234,11 +234,11 @@ __global__ void __launch_bounds__(kBlock, POLAR_SPMM_MINB) mk_spmm(const __grid_
     double dacc[CPL];
 #pragma unroll
     for (int v = 0; v < CPL; ++v) dacc[v] = 0.0;
-    heavy_chunk_pass<T, CPL, W, A>(
+    heavy_chunk_pass<T, CPL, W, A, true>(
         g, rg, wid, nw, P.d, ld, ld, on, s_idx[warp], chunk_part, P.hcount, hp,
         [&](int i, int cnt, auto& acc, auto& xi) {
           T yi[CPL];
-          finish_row_pre<T, CPL, false, A>(g, rg, i, cnt, shift, P.d, ld, acc, P.v, ld, xi, yi, on);
+          finish_row_pre<T, CPL, false, A, true>(g, rg, i, cnt, shift, P.d, ld, acc, P.v, ld, xi, yi, on);
           if (on)
 #pragma unroll
             for (int v = 0; v < CPL; ++v) dacc[v] += (double)xi[v] * (double)yi[v];
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kBlock, POLAR_SPMM_MINB) mk_spmm(const __grid_
         },
         [&](int i, int deg, auto& sum) {
           T xf[CPL], yi[CPL];
-          finish_row<T, CPL, false, A>(g, rg, i, deg, shift, P.d, ld, sum, P.v, ld, xf, yi, on);
+          finish_row<T, CPL, false, A, true>(g, rg, i, deg, shift, P.d, ld, sum, P.v, ld, xf, yi, on);
         });
     if (MODE == 1) {
       // heavy-only launch: partial d.v per CTA, reduced by the light launch's last CTA
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kBlock, POLAR_SPMM_MINB) mk_spmm(const __grid_
         T yv[CPL];
 #pragma unroll
         for (int v = 0; v < CPL; ++v) yv[v] = (T)fma((A)dg, (A)xi[v], -acc[v]);
-        vstore_hint<T, CPL>(P.v + (size_t)row * ld + rg.col, yv, hp.stream);
+        vstore_hint<T, CPL, true>(P.v + (size_t)row * ld + rg.col, yv, hp.stream);
 #pragma unroll
         for (int v = 0; v < CPL; ++v) acc[v] = (A)yv[v];
       }
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kBlock, POLAR_SPMM_MINB) mk_spmm(const __grid_
       sell_slice_pass_async<T, CPL, A>(g, rg, wid, nw, P.d, ld, on, hp, spmm_ring + (size_t)warp * kSellRingWarp,
                                        row_end);
     } else {
-      sell_slice_pass<T, CPL, A>(g, rg, wid, nw, P.d, ld, on, hp, row_end);
+      sell_slice_pass<T, CPL, A, true>(g, rg, wid, nw, P.d, ld, on, hp, row_end);
     }
     reduce_red_to_part(red, ld, P.part + (size_t)blockIdx.x * ld);
   } else {
@@ -319,12 +319,12 @@ __global__ void __launch_bounds__(kBlock, POLAR_SPMM_MINB) mk_spmm(const __grid_
       const int lo = __ldg(g.d_indptr + i), hi = __ldg(g.d_indptr + i + 1);
       if (hi - lo > g.heavy_thresh) continue;
       T xi[CPL], yi[CPL];
-      if (on) vload<T, CPL>(xi, P.d + (size_t)i * ld + rg.col);
+      if (on) vload<T, CPL, true>(xi, P.d + (size_t)i * ld + rg.col);
       A acc[CPL];
 #pragma unroll
       for (int v = 0; v < CPL; ++v) acc[v] = A(0);
-      gather_rows<T, CPL, W, A>(g, rg, lo, hi, P.d, ld, acc, on);
-      finish_row_pre<T, CPL, false, A>(g, rg, i, hi - lo, shift, P.d, ld, acc, P.v, ld, xi, yi, on);
+      gather_rows<T, CPL, W, A, true>(g, rg, lo, hi, P.d, ld, acc, on);
+      finish_row_pre<T, CPL, false, A, true>(g, rg, i, hi - lo, shift, P.d, ld, acc, P.v, ld, xi, yi, on);
       if (!on)
 #pragma unroll
         for (int v = 0; v < CPL; ++v) xi[v] = T(0);
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kBlock, POLAR_STREAM_MINB) mk_resid(const __gr
   }
   if (any_on) {
     T* hslot = P.hist + (size_t)slot * nA * ld;
-    constexpr int U = sizeof(T) == 4 ? POLAR_RESID_U32 : POLAR_RESID_U;
+    constexpr int U = sizeof(T) == 4 ? POLAR_RESID_U32 : (VEC >= 4 && POLAR_RESID_U > 1 ? POLAR_RESID_U / 2 : POLAR_RESID_U);
     for (long long e0 = tid; e0 < nvec; e0 += U * nth) {
       double rv[U][VEC];
       T vv[U][VEC];
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(kBlock, POLAR_STREAM_MINB) mk_resid(const __gr
         ii[u] = e < nvec ? (e >> lgG) : -1;
         if (ii[u] >= 0) {
           load_res<T, VEC>(P, rv[u], (size_t)ii[u] * ld + rg.col);
-          vload<T, VEC>(vv[u], P.v + (size_t)ii[u] * ld + rg.col);
+          vload<T, VEC, true>(vv[u], P.v + (size_t)ii[u] * ld + rg.col);
           ai[u] = __ldg(P.active_pos + ii[u]);
         }
       }
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(kBlock, POLAR_STREAM_MINB) mk_resid(const __gr
           racc[v] += rv[u][v] * rv[u][v];
           rt[v] = (T)rv[u][v];
         }
-        if (ai[u] >= 0) vstore_cs<T, VEC>(hslot + (size_t)ai[u] * ld + rg.col, rt);
+        if (ai[u] >= 0) vstore_cs<T, VEC, true>(hslot + (size_t)ai[u] * ld + rg.col, rt);
       }
     }
   }
@@ -508,8 +508,8 @@ __global__ void __launch_bounds__(kBlock, POLAR_STREAM_MINB) mk_dir(const __grid
     if (any_on) {
       const uint64_t pol_hot = l2_policy(P.l2_mode ? 1 : 0);
       const uint64_t pol_norm = l2_policy(0);
-      // FP64 r doubles the registers of a row item: fewer items in flight for wide FP32 rows
-      constexpr int U = (sizeof(T) == 4 && VEC >= 4 && POLAR_STREAM_U > 2) ? 2 : POLAR_STREAM_U;
+      // four FP64 columns take the registers of two row items of two
+      constexpr int U = (VEC >= 4 && POLAR_STREAM_U > 2) ? 2 : POLAR_STREAM_U;
       for (long long e0 = tid; e0 < nvec; e0 += U * nth) {
         double rv[U][VEC], dv[U][VEC];
         long long ii[U];
@@ -667,8 +667,12 @@ static int g_spmm_cpl_bytes = 0;  // 0: automatic
 
 template <typename T>
 static int spmm_cpl(int ld, int vec) {
-  // 32 bytes per lane for rows of 512 bytes or more, otherwise one 16-byte access
-  int bytes = g_spmm_cpl_bytes ? g_spmm_cpl_bytes : (ld * (int)sizeof(T) >= 512 ? 32 : 16);
+  // 32 bytes per lane (one 256-bit access) from 128-byte rows of FP64 and 512-byte rows of FP32 on,
+  // otherwise 16.  us per SpMM launch at n = 317,000, 16 -> 32 bytes: FP64 R = 8 47.3 -> 50.1,
+  // R = 16 68.8 -> 61.8, R = 32 120.5 -> 99.9; mixed R = 16 57.3 -> 75.0, R = 32 86.3 -> 92.6,
+  // R = 64 147.7 -> 142.8 but eight such solves at a time 85 -> 93 ms (FP32 lanes carry twice the
+  // FP64 sums), R = 128 267.9 -> 250.1; 64 bytes 368.9.
+  int bytes = g_spmm_cpl_bytes ? g_spmm_cpl_bytes : (ld * (int)sizeof(T) >= (sizeof(T) == 8 ? 128 : 512) ? 32 : 16);
   int cpl = bytes / (int)sizeof(T);
   if (cpl < vec) cpl = vec;
   if (cpl > ld) cpl = ld;
@@ -750,9 +754,16 @@ static int flush_grid(const SolvePrm<T>& P, size_t smem) {
   return g < nch ? nch : g;
 }
 
+// Columns per lane of the r and d updates of FP64 rows of 128 bytes or more (as in the SpMM): 32
+// bytes, one 256-bit access a vector (n = 317,000 R = 16: 35.3 -> 34.4 and 29.7 -> 28.0 us).
+template <typename T, int VEC>
+constexpr int stream_vec() {
+  return sizeof(T) == 8 && VEC == 2 ? 4 : VEC;
+}
+
 template <typename T, int VEC, bool W, int E>
 int mk_grid_max() {
-  int g = 0;
+  int g = occ_grid(mk_resid<T, stream_vec<T, VEC>()>, kBlock);
   for (int cpl = 1; cpl <= 16 / (int)(sizeof(T) / 4); cpl *= 2) {
     const int gc = spmm_grid<T, W>(cpl);
     g = g > gc ? g : gc;
@@ -793,6 +804,7 @@ struct MkSolver {
     double bytes;
     cudaEvent_t a, b;
   };
+  static constexpr int SV = stream_vec<T, VEC>();
   SolvePrm<T> P;
   cudaStream_t st = nullptr;
   cudaStream_t cs = nullptr;
@@ -842,8 +854,9 @@ struct MkSolver {
     const int cpl = spmm_cpl<T>(P.ld, VEC);
     if (spmm_merged<T, W>(cpl, P)) P.nbh = 0;
     const int g1 = scaled(spmm_grid<T, W>(cpl), f, 1);
-    const int g3 = scaled(occ_grid(mk_resid<T, VEC>, kBlock), f, 1);
-    const int g4 = scaled(occ_grid(mk_dir<T, VEC>, kBlock), f, 1);
+    const bool wide = SV > VEC && P.ld * sizeof(T) >= 128;
+    const int g3 = scaled(wide ? occ_grid(mk_resid<T, SV>, kBlock) : occ_grid(mk_resid<T, VEC>, kBlock), f, 1);
+    const int g4 = scaled(wide ? occ_grid(mk_dir<T, SV>, kBlock) : occ_grid(mk_dir<T, VEC>, kBlock), f, 1);
     s5 = flush_smem_for<T, E>(P);
     g5 = scaled(flush_grid<T, E>(P, s5), f, P.ld / flush_cw<T>(P.ld));
     // added edges: one thread per (row, column) up to one CTA per SM
@@ -890,8 +903,8 @@ struct MkSolver {
       if (P.nbh > 0) node(cs, KC_HEAVY, 0.0, [&](cudaStream_t x) { spmm_go<T, W>(1, cpl, g1, P, x); });
       node(cs, KC_SPMM, b_spmm, [&](cudaStream_t x) { spmm_go<T, W>(2, cpl, g1, P, x); });
       if (gx > 0) node(cs, KC_ADDED, b_added, [&](cudaStream_t x) { launch_k(mk_added<T>, gx, kBlock, 0, x, P); });
-      node(cs, KC_RESID, b_resid, [&](cudaStream_t x) { launch_k(mk_resid<T, VEC>, g3, kBlock, 0, x, P, k); });
-      node(cs, KC_DIR, b_dir, [&](cudaStream_t x) { launch_k(mk_dir<T, VEC>, g4, kBlock, 0, x, P, k); });
+      node(cs, KC_RESID, b_resid, [&](cudaStream_t x) { launch_k(wide ? mk_resid<T, SV> : mk_resid<T, VEC>, g3, kBlock, 0, x, P, k); });
+      node(cs, KC_DIR, b_dir, [&](cudaStream_t x) { launch_k(wide ? mk_dir<T, SV> : mk_dir<T, VEC>, g4, kBlock, 0, x, P, k); });
     }
     node(cs, KC_FLUSH, b_flush, [&](cudaStream_t x) { launch_k(mk_flush<T, E>, g5, kBlock, s5, x, P, 0); });
     e = cudaStreamEndCapture(cs, &graph);

@@ -115,7 +115,8 @@ POLAR_D GatherHints make_gather_hints(int mode, int hot_rows, const void* X = nu
 // partial(i, first, acc, xi): after a multi-chunk row's partial is stored (grp == 0, on);
 // fin(i, deg, sum): the last-arriving chunk with the row's combined sum (grp == 0).
 // xi is row i's own entries (loaded for grp == 0 when on).  s_idx: this warp's kChunkMax ints.
-template <typename T, int CPL, bool W, typename A, typename Single, typename Partial, typename Final>
+// W32: rows of X and of chunk_part are 32-byte aligned.
+template <typename T, int CPL, bool W, typename A, bool W32, typename Single, typename Partial, typename Final>
 POLAR_D void heavy_chunk_pass(const polar_graph& g, const RowGroup& rg, int wid, int nw, const T* X, int ldx, int ldp,
                               bool on, int* s_idx, A* chunk_part, int* hcount, const GatherHints& hp,
                               Single&& single, Partial&& partial, Final&& fin) {
@@ -131,7 +132,7 @@ POLAR_D void heavy_chunk_pass(const polar_graph& g, const RowGroup& rg, int wid,
     const int c0 = __ldg(g.d_hchunk_off + h), c1 = __ldg(g.d_hchunk_off + h + 1);
     const bool one = (c1 - c0) == 1;
     T xi[CPL];
-    if (on && grp == 0) vload<T, CPL>(xi, X + (size_t)i * ldx + rg.col);
+    if (on && grp == 0) vload<T, CPL, W32>(xi, X + (size_t)i * ldx + rg.col);
     const int cnt = hi - lo;
     __syncwarp();
 #pragma unroll
@@ -153,7 +154,7 @@ POLAR_D void heavy_chunk_pass(const polar_graph& g, const RowGroup& rg, int wid,
         if (on && u0 + uu < nu) {
           const int t = grp + gpw * (u0 + uu);
           const int j = s_idx[t];
-          vload_hint<T, CPL>(xv[uu], X + (size_t)j * ldx + rg.col, hp.row(j));
+          vload_hint<T, CPL, W32>(xv[uu], X + (size_t)j * ldx + rg.col, hp.row(j));
           wv[uu] = W ? (A)__ldg(g.d_wts + lo + t) : A(1);
         }
 #pragma unroll
@@ -171,7 +172,7 @@ POLAR_D void heavy_chunk_pass(const polar_graph& g, const RowGroup& rg, int wid,
       continue;
     }
     if (on && grp == 0) {
-      vstore<A, CPL>(chunk_part + (size_t)ch * ldp + rg.col, acc);
+      vstore<A, CPL, W32>(chunk_part + (size_t)ch * ldp + rg.col, acc);
       partial(i, ch == c0, acc, xi);
     }
     __threadfence();
@@ -206,7 +207,7 @@ POLAR_D void heavy_chunk_pass(const polar_graph& g, const RowGroup& rg, int wid,
 // Latency: a slice's work is a chain index load -> gathers -> accumulate per batch, so the
 // indices of the next batch (or of the next slice's first batch) are loaded while this
 // batch's gathers are in flight, and the row's own entries are loaded at the slice start.
-template <typename T, int CPL, typename A, typename RowEnd>
+template <typename T, int CPL, typename A, bool W32, typename RowEnd>
 POLAR_D void sell_slice_pass(const polar_graph& g, const RowGroup& rg, int wid, int nw, const T* X, int ldx, bool on,
                              const GatherHints& hp, RowEnd&& row_end) {
   constexpr int LB = CPL * (int)sizeof(T);
@@ -238,7 +239,7 @@ POLAR_D void sell_slice_pass(const polar_graph& g, const RowGroup& rg, int wid, 
     if (sn < g.nsl) fetch_desc(sn, off_n, w_n, row_n);
     const bool go = row >= 0 && on;
     T xi[CPL];
-    if (go) vload_hint<T, CPL>(xi, X + (size_t)row * ldx + rg.col, hp.row(row));
+    if (go) vload_hint<T, CPL, W32>(xi, X + (size_t)row * ldx + rg.col, hp.row(row));
     A acc[CPL];
 #pragma unroll
     for (int v = 0; v < CPL; ++v) acc[v] = A(0);
@@ -251,7 +252,7 @@ POLAR_D void sell_slice_pass(const polar_graph& g, const RowGroup& rg, int wid, 
       T xv[U][CPL];
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (go && jj[u] >= 0) vload_hint<T, CPL>(xv[u], X + (size_t)jj[u] * ldx + rg.col, hp.row(jj[u]));
+        if (go && jj[u] >= 0) vload_hint<T, CPL, W32>(xv[u], X + (size_t)jj[u] * ldx + rg.col, hp.row(jj[u]));
       int jn[U];
       if (k + U < w)
         fetch_idx(off, w, k + U, jn);

@@ -92,16 +92,19 @@ POLAR_D uint64_t row_policy(const SolvePrm<T>& P, long long i, uint64_t hot, uin
   return i < P.hot_rows ? hot : cold;
 }
 
+// The workspace's row vectors start 256-byte aligned and their rows are a power of two of at least
+// one vector, so 32-byte row items take 256-bit accesses.
+//
 // Residual of one row item: the FP64 r, or the FP32 residual when r32 is set.
 template <typename T, int VEC>
 POLAR_D void load_res(const SolvePrm<T>& P, double (&out)[VEC], size_t o) {
   if (P.r32) {
     float t[VEC];
-    vload<float, VEC>(t, P.r32 + o);
+    vload<float, VEC, true>(t, P.r32 + o);
 #pragma unroll
     for (int v = 0; v < VEC; ++v) out[v] = (double)t[v];
   } else {
-    vload<double, VEC>(out, P.r + o);
+    vload<double, VEC, true>(out, P.r + o);
   }
 }
 
@@ -116,9 +119,9 @@ POLAR_D void store_res(const SolvePrm<T>& P, double (&x)[VEC], size_t o) {
       t[v] = (float)x[v];
       x[v] = (double)t[v];
     }
-    vstore<float, VEC>(P.r32 + o, t);
+    vstore<float, VEC, true>(P.r32 + o, t);
   } else {
-    vstore<double, VEC>(P.r + o, x);
+    vstore<double, VEC, true>(P.r + o, x);
   }
 }
 
@@ -127,12 +130,12 @@ POLAR_D void store_res(const SolvePrm<T>& P, double (&x)[VEC], size_t o) {
 template <typename T, int VEC>
 POLAR_D void load_dir(const SolvePrm<T>& P, double (&out)[VEC], size_t o) {
   T hi[VEC];
-  vload<T, VEC>(hi, P.d + o);
+  vload<T, VEC, true>(hi, P.d + o);
 #pragma unroll
   for (int v = 0; v < VEC; ++v) out[v] = (double)hi[v];
   if (P.dlo) {
     float lo[VEC];
-    vload<float, VEC>(lo, P.dlo + o);
+    vload<float, VEC, true>(lo, P.dlo + o);
 #pragma unroll
     for (int v = 0; v < VEC; ++v) out[v] += (double)lo[v];
   }
@@ -143,12 +146,12 @@ POLAR_D void store_dir(const SolvePrm<T>& P, const double (&in)[VEC], size_t o) 
   T hi[VEC];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) hi[v] = (T)in[v];
-  vstore<T, VEC>(P.d + o, hi);
+  vstore<T, VEC, true>(P.d + o, hi);
   if (P.dlo) {
     float lo[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) lo[v] = (float)(in[v] - (double)hi[v]);
-    vstore<float, VEC>(P.dlo + o, lo);
+    vstore<float, VEC, true>(P.dlo + o, lo);
   }
 }
 
@@ -159,12 +162,12 @@ POLAR_D void store_dir_hint(const SolvePrm<T>& P, const double (&in)[VEC], size_
   T hi[VEC];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) hi[v] = (T)in[v];
-  vstore_hint<T, VEC>(P.d + o, hi, dpol);
+  vstore_hint<T, VEC, true>(P.d + o, hi, dpol);
   if (P.dlo) {
     float lo[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) lo[v] = (float)(in[v] - (double)hi[v]);
-    vstore_hint<float, VEC>(P.dlo + o, lo, lopol);
+    vstore_hint<float, VEC, true>(P.dlo + o, lo, lopol);
   }
 }
 
@@ -186,31 +189,52 @@ POLAR_D void reduce_cols_to_part(double (&acc)[VEC], int G, int ld, double* red,
   }
 }
 
-// Sum of per-CTA partials part[b][c] over b in a fixed order (deterministic).
+// Sum of per-CTA partials part[b][c] over b in a fixed order (deterministic).  One CTA runs it
+// while the GPU waits, so it is all latency: a thread takes two columns (one when ld is 1) of a strip
+// of blocks, ten 16-byte loads issued before the adds, and the strips are summed in two short
+// rounds.  tmp: kWarps * kMaxLd doubles.
 POLAR_D void reduce_partials(const double* part, int nblk, int ld, double* tmp, double* out) {
-  const int S = blockDim.x / ld;
-  const int t = threadIdx.x, c = t % ld, s = t / ld;
-  if (s < S) {
-    // strip s sums blocks s, s + S, ... in that order; eight loads are issued before the
-    // adds so the strip costs about one L2 round trip per eight partials
-    constexpr int B = 8;
-    double acc = 0.0;
+  static_assert(kBlock * 2 + 8 * kMaxLd <= kWarps * kMaxLd, "strips and their partial sums fit tmp");
+  const int t = threadIdx.x, V = ld > 1 ? 2 : 1, hl = ld / V;
+  const int S = (int)blockDim.x / hl, c = V * (t % hl), s = t / hl;
+  {
+    constexpr int B = 10;
+    double a0 = 0.0, a1 = 0.0;
     for (int b0 = s; b0 < nblk; b0 += B * S) {
-      double v[B];
+      double2 v[B];
 #pragma unroll
       for (int u = 0; u < B; ++u) {
         const int b = b0 + u * S;
-        v[u] = b < nblk ? __ldcg(part + (size_t)b * ld + c) : 0.0;
+        v[u] = make_double2(0.0, 0.0);
+        if (b < nblk) {
+          if (V == 2) v[u] = __ldcg(reinterpret_cast<const double2*>(part + (size_t)b * ld + c));
+          else v[u].x = __ldcg(part + b);
+        }
       }
 #pragma unroll
-      for (int u = 0; u < B; ++u) acc += v[u];
+      for (int u = 0; u < B; ++u) {
+        a0 += v[u].x;
+        a1 += v[u].y;
+      }
     }
-    tmp[s * ld + c] = acc;
+    tmp[s * ld + c] = a0;
+    if (V == 2) tmp[s * ld + c + 1] = a1;
+  }
+  __syncthreads();
+  constexpr int Q = 8;
+  double* tmp2 = tmp + 2 * kBlock;
+  for (int i = t; i < Q * ld; i += blockDim.x) {
+    const int q = i / ld, cc = i - q * ld;
+    double acc = 0.0;
+#pragma unroll 8
+    for (int s2 = q; s2 < S; s2 += Q) acc += tmp[s2 * ld + cc];
+    tmp2[i] = acc;
   }
   __syncthreads();
   if (t < ld) {
     double acc = 0.0;
-    for (int s2 = 0; s2 < S; ++s2) acc += tmp[s2 * ld + t];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) acc += tmp2[q * ld + t];
     out[t] = acc;
   }
   __syncthreads();

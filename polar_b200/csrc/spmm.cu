@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(512, POLAR_PANEL_MINB) spmm_panel_kernel(polar
 // Sliced-ELL path (unweighted graphs with the layout for this width): the solver's SpMM
 // passes with the standalone row finish (diagonal, shift and the greedy's added edges per
 // row), FP64 row sums, the same L2 policies.  R == ld, a power of two.
-template <typename T, int CPL>
+template <typename T, int CPL, bool W32>
 __global__ void __launch_bounds__(512, 2) spmm_sell_kernel(polar_graph g, int ld, double shift, const T* X,
                                                            int ldx, T* Y, int ldy, double* part, int* hcount,
                                                            int l2_mode, int hot_rows) {
@@ -101,16 +101,16 @@ __global__ void __launch_bounds__(512, 2) spmm_sell_kernel(polar_graph g, int ld
   const int wid = blockIdx.x * 16 + warp;
   const int nw = gridDim.x * 16;
   const GatherHints hp = make_gather_hints(l2_mode, hot_rows, X, (size_t)ldx * sizeof(T), g.n);
-  heavy_chunk_pass<T, CPL, false, A>(
+  heavy_chunk_pass<T, CPL, false, A, W32>(
       g, rg, wid, nw, X, ldx, ld, true, s_idx[warp], part, hcount, hp,
       [&](int i, int cnt, auto& acc, auto& xi) {
         T yi[CPL];
-        finish_row_pre<T, CPL, true, A>(g, rg, i, cnt, shift, X, ldx, acc, Y, ldy, xi, yi, true);
+        finish_row_pre<T, CPL, true, A, W32>(g, rg, i, cnt, shift, X, ldx, acc, Y, ldy, xi, yi, true);
       },
       [&](int, bool, auto&, auto&) {},
       [&](int i, int deg, auto& sum) {
         T xf[CPL], yi[CPL];
-        finish_row<T, CPL, true, A>(g, rg, i, deg, shift, X, ldx, sum, Y, ldy, xf, yi, true);
+        finish_row<T, CPL, true, A, W32>(g, rg, i, deg, shift, X, ldx, sum, Y, ldy, xf, yi, true);
       });
   auto row_end = [&](int row, int deg, auto& acc, auto& xi, bool go) {
     if (!go) return;
@@ -119,19 +119,19 @@ __global__ void __launch_bounds__(512, 2) spmm_sell_kernel(polar_graph g, int ld
     T yv[CPL];
 #pragma unroll
     for (int v = 0; v < CPL; ++v) yv[v] = (T)fma((A)dg, (A)xi[v], -acc[v]);
-    vstore_hint<T, CPL>(Y + (size_t)row * ldy + rg.col, yv, hp.stream);
+    vstore_hint<T, CPL, W32>(Y + (size_t)row * ldy + rg.col, yv, hp.stream);
   };
   if constexpr (POLAR_SELL_ASYNC != 0 && (CPL * sizeof(T)) % 16 == 0) {
     extern __shared__ __align__(16) unsigned char sell_ring[];
     sell_slice_pass_async<T, CPL, A>(g, rg, wid, nw, X, ldx, true, hp,
                                      sell_ring + (size_t)warp * POLAR_SELL_STAGES * POLAR_SELL_BYTES * 32, row_end);
   } else {
-    sell_slice_pass<T, CPL, A>(g, rg, wid, nw, X, ldx, true, hp, row_end);
+    sell_slice_pass<T, CPL, A, W32>(g, rg, wid, nw, X, ldx, true, hp, row_end);
   }
 }
 
-template <typename T, int CPL>
-static int launch_spmm_sell(const polar_graph& g, int ld, double shift, const void* X, int ldx, void* Y, int ldy,
+template <typename T, int CPL, bool W32>
+static int launch_spmm_sell_as(const polar_graph& g, int ld, double shift, const void* X, int ldx, void* Y, int ldy,
                             void* scratch, int precision, cudaStream_t st) {
   double* part = reinterpret_cast<double*>(scratch);
   int* hcount = reinterpret_cast<int*>(reinterpret_cast<char*>(scratch) + spmm_counter_offset(&g, precision));
@@ -140,20 +140,34 @@ static int launch_spmm_sell(const polar_graph& g, int ld, double shift, const vo
                           ? (size_t)16 * POLAR_SELL_STAGES * POLAR_SELL_BYTES * 32 : 0;
   static bool attr = false;
   if (!attr && ring > 0)
-    cudaFuncSetAttribute(spmm_sell_kernel<T, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
+    cudaFuncSetAttribute(spmm_sell_kernel<T, CPL, W32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
   attr = true;
   int dev = 0, sms = 0, nb = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, spmm_sell_kernel<T, CPL>, 512, ring);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, spmm_sell_kernel<T, CPL, W32>, 512, ring);
   if (nb < 1) nb = 1;
   const long long hot = (long long)(l2_hot_bytes_setting() / ((size_t)ld * sizeof(T)));
-  spmm_sell_kernel<T, CPL><<<nb * sms, 512, ring, st>>>(g, ld, shift, (const T*)X, ldx, (T*)Y, ldy, part, hcount,
+  spmm_sell_kernel<T, CPL, W32><<<nb * sms, 512, ring, st>>>(g, ld, shift, (const T*)X, ldx, (T*)Y, ldy, part, hcount,
                                                          l2_mode_setting(), (int)(hot < g.n ? hot : g.n));
   count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_cuda_error("spmm launch", e);
   return POLAR_OK;
+}
+
+// 32 bytes or more per lane: 256-bit accesses when every row of the blocks (and the chunk
+// partials) allows them.
+template <typename T, int CPL>
+static int launch_spmm_sell(const polar_graph& g, int ld, double shift, const void* X, int ldx, void* Y, int ldy,
+                            void* scratch, int precision, cudaStream_t st) {
+  if constexpr (takes32<T, CPL, true>()) {
+    const size_t es = sizeof(T);
+    if ((uintptr_t)X % 32 == 0 && (uintptr_t)Y % 32 == 0 && (uintptr_t)scratch % 32 == 0 && (size_t)ldx * es % 32 == 0 &&
+        (size_t)ldy * es % 32 == 0)
+      return launch_spmm_sell_as<T, CPL, true>(g, ld, shift, X, ldx, Y, ldy, scratch, precision, st);
+  }
+  return launch_spmm_sell_as<T, CPL, false>(g, ld, shift, X, ldx, Y, ldy, scratch, precision, st);
 }
 
 // The sliced-ELL launch for this call, or nothing (used = false) when the row-loop

@@ -91,7 +91,8 @@ def msolve_batch(ops, Ws, taus, actives, tol, maxit=100000, track=False, *, prec
         h = torch.zeros((p, R), dtype=torch.float64, device=dev) if track else None
         iters = torch.zeros(R, dtype=torch.int64, device=dev)
         thresh, chunk = heavy_partition(G, prec, R)
-        gs = ops[b].struct(heavy_thresh=thresh, sell_rows=lib.polar_sell_rows(prec, R), chunk=chunk)
+        S = lib.polar_sell_rows(prec, R)
+        gs = ops[b].struct(heavy_thresh=thresh, sell_rows=S, chunk=chunk, row_blocks=S == 0)
         need = lib.polar_msolve_batch_workspace_bytes(gs, prec, R, p, nA)
         ws = _workspace(b, need, dev)
         q = probs[b]

@@ -89,28 +89,31 @@ __global__ void __launch_bounds__(512, POLAR_PANEL_MINB) spmm_panel_kernel(polar
 
 // Sliced-ELL path (unweighted graphs with the layout for this width): the solver's SpMM
 // passes with the standalone row finish (diagonal, shift and the greedy's added edges per
-// row), FP64 row sums, the same L2 policies.  R == ld, a power of two.
+// row), FP64 row sums, the same L2 policies.  Widths that are not a power of two take it too
+// (n = 10^6 FP64, row-loop kernel -> this: R = 20 341 -> 285 us, R = 28 381 -> 327).  ld: R rounded up to a power of two; lanes whose
+// columns lie beyond R (whole lanes only) take part in the indices and issue no loads.
 template <typename T, int CPL, bool W32>
-__global__ void __launch_bounds__(512, 2) spmm_sell_kernel(polar_graph g, int ld, double shift, const T* X,
+__global__ void __launch_bounds__(512, 2) spmm_sell_kernel(polar_graph g, int R, int ld, double shift, const T* X,
                                                            int ldx, T* Y, int ldy, double* part, int* hcount,
                                                            int l2_mode, int hot_rows) {
   using A = double;
   __shared__ int s_idx[16][kChunkMax];
   const RowGroup rg = make_row_group<CPL>(ld);
+  const bool on = rg.col < R;
   const int warp = threadIdx.x >> 5;
   const int wid = blockIdx.x * 16 + warp;
   const int nw = gridDim.x * 16;
   const GatherHints hp = make_gather_hints(l2_mode, hot_rows, X, (size_t)ldx * sizeof(T), g.n);
   heavy_chunk_pass<T, CPL, false, A, W32>(
-      g, rg, wid, nw, X, ldx, ld, true, s_idx[warp], part, hcount, hp,
+      g, rg, wid, nw, X, ldx, ld, on, s_idx[warp], part, hcount, hp,
       [&](int i, int cnt, auto& acc, auto& xi) {
         T yi[CPL];
-        finish_row_pre<T, CPL, true, A, W32>(g, rg, i, cnt, shift, X, ldx, acc, Y, ldy, xi, yi, true);
+        finish_row_pre<T, CPL, true, A, W32>(g, rg, i, cnt, shift, X, ldx, acc, Y, ldy, xi, yi, on);
       },
       [&](int, bool, auto&, auto&) {},
       [&](int i, int deg, auto& sum) {
         T xf[CPL], yi[CPL];
-        finish_row<T, CPL, true, A, W32>(g, rg, i, deg, shift, X, ldx, sum, Y, ldy, xf, yi, true);
+        finish_row<T, CPL, true, A, W32>(g, rg, i, deg, shift, X, ldx, sum, Y, ldy, xf, yi, on);
       });
   auto row_end = [&](int row, int deg, auto& acc, auto& xi, bool go) {
     if (!go) return;
@@ -123,15 +126,15 @@ __global__ void __launch_bounds__(512, 2) spmm_sell_kernel(polar_graph g, int ld
   };
   if constexpr (POLAR_SELL_ASYNC != 0 && (CPL * sizeof(T)) % 16 == 0) {
     extern __shared__ __align__(16) unsigned char sell_ring[];
-    sell_slice_pass_async<T, CPL, A>(g, rg, wid, nw, X, ldx, true, hp,
+    sell_slice_pass_async<T, CPL, A>(g, rg, wid, nw, X, ldx, on, hp,
                                      sell_ring + (size_t)warp * POLAR_SELL_STAGES * POLAR_SELL_BYTES * 32, row_end);
   } else {
-    sell_slice_pass<T, CPL, A, W32>(g, rg, wid, nw, X, ldx, true, hp, row_end);
+    sell_slice_pass<T, CPL, A, W32>(g, rg, wid, nw, X, ldx, on, hp, row_end);
   }
 }
 
 template <typename T, int CPL, bool W32>
-static int launch_spmm_sell_as(const polar_graph& g, int ld, double shift, const void* X, int ldx, void* Y, int ldy,
+static int launch_spmm_sell_as(const polar_graph& g, int R, int ld, double shift, const void* X, int ldx, void* Y, int ldy,
                             void* scratch, int precision, cudaStream_t st) {
   double* part = reinterpret_cast<double*>(scratch);
   int* hcount = reinterpret_cast<int*>(reinterpret_cast<char*>(scratch) + spmm_counter_offset(&g, precision));
@@ -148,7 +151,7 @@ static int launch_spmm_sell_as(const polar_graph& g, int ld, double shift, const
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, spmm_sell_kernel<T, CPL, W32>, 512, ring);
   if (nb < 1) nb = 1;
   const long long hot = (long long)(l2_hot_bytes_setting() / ((size_t)ld * sizeof(T)));
-  spmm_sell_kernel<T, CPL, W32><<<nb * sms, 512, ring, st>>>(g, ld, shift, (const T*)X, ldx, (T*)Y, ldy, part, hcount,
+  spmm_sell_kernel<T, CPL, W32><<<nb * sms, 512, ring, st>>>(g, R, ld, shift, (const T*)X, ldx, (T*)Y, ldy, part, hcount,
                                                          l2_mode_setting(), (int)(hot < g.n ? hot : g.n));
   count_launch();
   cudaError_t e = cudaGetLastError();
@@ -159,38 +162,39 @@ static int launch_spmm_sell_as(const polar_graph& g, int ld, double shift, const
 // 32 bytes or more per lane: 256-bit accesses when every row of the blocks (and the chunk
 // partials) allows them.
 template <typename T, int CPL>
-static int launch_spmm_sell(const polar_graph& g, int ld, double shift, const void* X, int ldx, void* Y, int ldy,
+static int launch_spmm_sell(const polar_graph& g, int R, int ld, double shift, const void* X, int ldx, void* Y, int ldy,
                             void* scratch, int precision, cudaStream_t st) {
   if constexpr (takes32<T, CPL, true>()) {
     const size_t es = sizeof(T);
     if ((uintptr_t)X % 32 == 0 && (uintptr_t)Y % 32 == 0 && (uintptr_t)scratch % 32 == 0 && (size_t)ldx * es % 32 == 0 &&
         (size_t)ldy * es % 32 == 0)
-      return launch_spmm_sell_as<T, CPL, true>(g, ld, shift, X, ldx, Y, ldy, scratch, precision, st);
+      return launch_spmm_sell_as<T, CPL, true>(g, R, ld, shift, X, ldx, Y, ldy, scratch, precision, st);
   }
-  return launch_spmm_sell_as<T, CPL, false>(g, ld, shift, X, ldx, Y, ldy, scratch, precision, st);
+  return launch_spmm_sell_as<T, CPL, false>(g, R, ld, shift, X, ldx, Y, ldy, scratch, precision, st);
 }
 
 // The sliced-ELL launch for this call, or nothing (used = false) when the row-loop
-// kernels apply: weighted graphs, no layout for this width, widths that are not a power of
-// two, or blocks that are not 16-byte aligned.
+// kernels apply: weighted graphs, no layout for this width, widths that leave a lane part of its
+// columns, or blocks that are not 16-byte aligned.
 template <typename T>
 static int try_spmm_sell(const polar_graph& g, int precision, int R, double shift, const void* X, int ldx, void* Y,
                          int ldy, void* scratch, cudaStream_t st, bool* used) {
   *used = false;
   const int vmin = 16 / (int)sizeof(T);  // one 16-byte vector per lane at least
-  if (g.d_wts || g.nsl <= 0 || R < vmin || (R & (R - 1)) != 0) return POLAR_OK;
-  const int lanes = mk_spmm_lanes(precision, R);
-  const int cpl = R / lanes;
-  if (g.sell_s != 32 / lanes) return POLAR_OK;
+  if (g.d_wts || g.nsl <= 0 || R < vmin) return POLAR_OK;
+  const int ld = next_pow2(R);
+  const int lanes = mk_spmm_lanes(precision, ld);
+  const int cpl = ld / lanes;
+  if (g.sell_s != 32 / lanes || R % cpl != 0) return POLAR_OK;
   const size_t es = sizeof(T);
   if ((uintptr_t)X % 16 || (uintptr_t)Y % 16 || ((size_t)ldx * es) % 16 || ((size_t)ldy * es) % 16) return POLAR_OK;
   *used = true;
   switch (cpl) {
-    case 2: return launch_spmm_sell<T, 2>(g, R, shift, X, ldx, Y, ldy, scratch, precision, st);
-    case 4: return launch_spmm_sell<T, 4>(g, R, shift, X, ldx, Y, ldy, scratch, precision, st);
-    case 8: return launch_spmm_sell<T, 8>(g, R, shift, X, ldx, Y, ldy, scratch, precision, st);
+    case 2: return launch_spmm_sell<T, 2>(g, R, ld, shift, X, ldx, Y, ldy, scratch, precision, st);
+    case 4: return launch_spmm_sell<T, 4>(g, R, ld, shift, X, ldx, Y, ldy, scratch, precision, st);
+    case 8: return launch_spmm_sell<T, 8>(g, R, ld, shift, X, ldx, Y, ldy, scratch, precision, st);
     case 16:
-      if (sizeof(T) == 4) return launch_spmm_sell<T, 16>(g, R, shift, X, ldx, Y, ldy, scratch, precision, st);
+      if (sizeof(T) == 4) return launch_spmm_sell<T, 16>(g, R, ld, shift, X, ldx, Y, ldy, scratch, precision, st);
       break;
   }
   *used = false;

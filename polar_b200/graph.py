@@ -250,15 +250,45 @@ class Graph:
         self.nheavy, self.nchunks = hv["nheavy"], hv["nchunks"]
         self.hrow, self.hchunk_off = hv["hrow"], hv["hchunk_off"]
         self.chunk_row, self.chunk_lo, self.chunk_hi = hv["chunk_row"], hv["chunk_lo"], hv["chunk_hi"]
-        self.rowblk_h, self.nrb, self.rowblk = hv["rowblk_h"], hv["nrb"], hv["rowblk"]
+        if self.n < 1_000_000:  # and the finer one that applies and solves of most widths take
+            t, ch = self._fine_partition(0)
+            if t < self.heavy_thresh:
+                self._heavy_parts(t, ch)
+
+    def _fine_partition(self, row_bytes):
+        """(threshold, chunk) of an apply with rows of that many bytes."""
+        if self.n < 200_000 or 0 < row_bytes <= 32:
+            return 32, 64
+        return (64 if self.n < 1_000_000 else self.heavy_thresh), 128
+
+    def _row_blocks(self, hv):
+        """Row blocks of a partition, built when a kernel first streams through them (the
+        sliced-ELL kernels do not; 10 ms on the host at n = 317,000)."""
+        if "nrb" not in hv:
+            rb = row_blocks(self._indptr_h, hv["thresh"])
+            hv.update(rowblk_h=rb, rowblk=_i32(rb.ravel() if len(rb) else np.zeros(2, np.int32), self.device),
+                      nrb=len(rb))
+        return hv
+
+    @property
+    def rowblk_h(self):
+        return self._row_blocks(self._heavy_parts(self.heavy_thresh))["rowblk_h"]
+
+    @property
+    def nrb(self):
+        return self._row_blocks(self._heavy_parts(self.heavy_thresh))["nrb"]
+
+    @property
+    def rowblk(self):
+        return self._row_blocks(self._heavy_parts(self.heavy_thresh))["rowblk"]
 
     def _heavy_parts(self, thresh, chunk=None):
         ch = self.CHUNK if chunk is None else min(int(chunk), self.CHUNK)
         if (thresh, ch) in self._heavy:
             return self._heavy[thresh, ch]
-        degs = np.diff(self._indptr_h.astype(np.int64))
+        degs = np.diff(self._indptr_h)
         hrow = np.flatnonzero(degs > thresh).astype(np.int32)
-        nch = -(-degs[hrow] // ch) if len(hrow) else np.zeros(0, np.int64)
+        nch = -(-degs[hrow].astype(np.int64) // ch)
         off = np.zeros(len(hrow) + 1, np.int64)
         off[1:] = np.cumsum(nch)
         total = int(off[-1])
@@ -270,9 +300,7 @@ class Graph:
         c_hi = np.minimum(c_lo + ch, np.repeat(hi, nch))
         dev = self.device
         one = np.zeros(1, np.int32)
-        rb = row_blocks(self._indptr_h, thresh)
-        hv = dict(thresh=thresh, nheavy=len(hrow), nchunks=total, rowblk_h=rb, nrb=len(rb),
-                  rowblk=_i32(rb.ravel() if len(rb) else np.zeros(2, np.int32), dev),
+        hv = dict(thresh=thresh, nheavy=len(hrow), nchunks=total,
                   hrow=_i32(hrow if len(hrow) else one, dev), hchunk_off=_i32(off, dev),
                   chunk_row=_i32(chunk_row if total else one, dev), chunk_lo=_i32(c_lo if total else one, dev),
                   chunk_hi=_i32(c_hi if total else one, dev))
@@ -303,12 +331,13 @@ class Graph:
                                              idx=_i32(sidx if len(sidx) else np.zeros(1, np.int32), dev))
         return self._sell_cache[key]
 
-    def struct(self, extra=None, heavy_thresh=None, sell_rows=0, chunk=None):
+    def struct(self, extra=None, heavy_thresh=None, sell_rows=0, chunk=None, row_blocks=True):
         """ctypes polar_graph for this graph (plus an Op's added edges), with the heavy-row
         partition for `heavy_thresh` (default: the graph's own threshold) in chunks of at most
         `chunk` neighbours (default CHUNK) and, when
         sell_rows > 0 (unweighted graphs), the sliced-ELL layout of the light rows for
-        warps of sell_rows rows."""
+        warps of sell_rows rows.  row_blocks=False leaves out the row blocks, for calls that only
+        reach the sliced-ELL kernels."""
         hv = self._heavy_parts(self.heavy_thresh if heavy_thresh is None else int(heavy_thresh), chunk)
         s = _lib.PolarGraph()
         s.nsl = 0
@@ -336,8 +365,10 @@ class Graph:
         s.d_chunk_row = hv["chunk_row"].data_ptr()
         s.d_chunk_lo = hv["chunk_lo"].data_ptr()
         s.d_chunk_hi = hv["chunk_hi"].data_ptr()
-        s.nrb = hv["nrb"]
-        s.d_rowblk = hv["rowblk"].data_ptr()
+        if row_blocks:
+            self._row_blocks(hv)
+            s.nrb = hv["nrb"]
+            s.d_rowblk = hv["rowblk"].data_ptr()
         if extra is not None:
             extra.fill(s)
         return s
@@ -413,8 +444,40 @@ class Op:
         self.B.append(b)
         self._added.add(a, b, float(w))
 
-    def struct(self, heavy_thresh=None, sell_rows=0, chunk=None):
-        return self.G.struct(self._added, heavy_thresh=heavy_thresh, sell_rows=sell_rows, chunk=chunk)
+    def struct(self, heavy_thresh=None, sell_rows=0, chunk=None, row_blocks=True):
+        return self.G.struct(self._added, heavy_thresh=heavy_thresh, sell_rows=sell_rows, chunk=chunk,
+                             row_blocks=row_blocks)
+
+    def _struct_for(self, lib, prec, R):
+        """The graph as an apply of width R takes it.
+
+        Rows: unweighted graphs whose rows are whole 16-byte vectors take the solver's sliced-ELL
+        layout.  Heavy-row partition: below a million rows, or with rows of at most 32 bytes, a
+        launch ends with its longest chain of gathers, so long rows are cut finer than the
+        graph's 256 neighbours (us per FP64 apply, 256 -> this: n = 20,000 R = 3 66 -> 23, R = 20
+        51 -> 20; n = 317,000 R = 1 64 -> 25, R = 14 95 -> 51, R = 16 86 -> 51, R = 20 99 -> 84, R = 64
+        257 -> 178; n = 10^6 R = 1 84 -> 43, but R = 28 381 -> 397).  The panel kernel (weighted
+        graphs at powers of two) streams through row blocks and keeps the graph's partition."""
+        vec = 4 if prec == _lib.POLAR_MIXED else 2
+        whole = R % vec == 0
+        sell = 0 if self.G.weighted or not whole else lib.polar_sell_rows(prec, R)
+        if sell == 0 and whole and R & (R - 1) == 0:
+            return self.struct()
+        thresh, chunk = self.G._fine_partition(R * (16 // vec))
+        if self.G.heavy_thresh <= thresh:
+            return self.struct(sell_rows=sell)
+        return self.struct(heavy_thresh=thresh, sell_rows=sell, chunk=chunk, row_blocks=False)
+
+    def _scratch_for(self, lib, g, prec, maxc, stream):
+        """Chunk partials and counters of `g`'s heavy-row partition: both their size and the
+        place of the counters follow from its numbers of chunks and rows."""
+        key = (prec, self.G.device.index, g.nchunks, g.nheavy)
+        if key not in self._scratch:
+            nb = lib.polar_spmm_scratch_bytes(g, prec, maxc)
+            buf = torch.empty(max(nb, 256), dtype=torch.uint8, device=self.G.device)
+            _lib.check(lib.polar_spmm_scratch_init(g, prec, maxc, buf.data_ptr(), stream), "spmm scratch")
+            self._scratch[key] = buf
+        return self._scratch[key]
 
     def __call__(self, x, shift=0.0):
         """Apply to an (n, R) or (n,) float64/float32 CUDA tensor; returns a new tensor."""
@@ -431,21 +494,12 @@ class Op:
         Y = torch.empty_like(X)
         lib = _lib.load()
         stream = torch.cuda.current_stream(X.device).cuda_stream
-        g = self.struct()
-        key = (prec, X.device.index)
-        if key not in self._scratch:
-            nb = lib.polar_spmm_scratch_bytes(g, prec, maxc)
-            buf = torch.empty(max(nb, 256), dtype=torch.uint8, device=X.device)
-            _lib.check(lib.polar_spmm_scratch_init(g, prec, maxc, buf.data_ptr(), stream), "spmm scratch")
-            self._scratch[key] = buf
-        scratch = self._scratch[key]
         for lo in range(0, R, maxc):
             hi = min(R, lo + maxc)
             xs = X[:, lo:hi]
             ys = Y[:, lo:hi]
-            # unweighted graphs: the sliced-ELL layout of the solver for this width (the
-            # library uses it when the width is a power of two)
-            gw = self.struct(sell_rows=lib.polar_sell_rows(prec, hi - lo)) if not self.G.weighted else g
-            _lib.check(lib.polar_spmm(gw, prec, hi - lo, float(shift), xs.data_ptr(), R, ys.data_ptr(), R,
+            g = self._struct_for(lib, prec, hi - lo)
+            scratch = self._scratch_for(lib, g, prec, maxc, stream)
+            _lib.check(lib.polar_spmm(g, prec, hi - lo, float(shift), xs.data_ptr(), R, ys.data_ptr(), R,
                                       scratch.data_ptr(), stream), "polar_spmm")
         return Y.reshape(-1) if squeeze else Y

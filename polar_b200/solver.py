@@ -166,9 +166,10 @@ def msolve(op, W, tau, active, tol, maxit=100000, track=False, counter=None, *, 
             lib.polar_set_sell(cfg[1])
         try:
             thresh, chunk = heavy_partition(G, prec, r)
+            S = lib.polar_sell_rows(prec, r)
             if cfg is not None:
                 thresh = cfg[2]
-            g = op.struct(heavy_thresh=thresh, sell_rows=lib.polar_sell_rows(prec, r), chunk=chunk)
+            g = op.struct(heavy_thresh=thresh, sell_rows=S, chunk=chunk, row_blocks=S == 0)
             need = lib.polar_msolve_workspace_bytes(g, prec, r, p, nA)
             ws = workspace(need, dev)
             hpart = torch.zeros((p, r), dtype=torch.float64, device=dev) if track else None

@@ -76,3 +76,29 @@ def test_apply_at_any_16_bytes(prec, R):
     bound = 1e-14 if prec == "fp64" else 2e-7
     for v in (x, x.clone()):
         assert float((op(v).double() - want).abs().max() / scale) < bound
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("own", [256, 8])  # the graph's own partition: coarser and finer than the rule's
+@pytest.mark.parametrize("R", [1, 2, 3, 4, 12, 14, 16, 20, 28, 31, 60])
+def test_apply_partitions(prec, weighted, own, R):
+    import torch
+    import polar_b200 as pg
+    n = 5000
+    E = chung_lu(n, 9.0, 2.1, 3, min_degree=1)  # rows of up to a few hundred neighbours
+    w = np.random.default_rng(1).uniform(0.5, 1.5, len(E)) if weighted else None
+    G = pg.Graph(n, E, 5e-1, weights=w, heavy_thresh=own)
+    op = pg.Op(G)
+    op.add(3, n - 1, 0.7)
+    dt = torch.float64 if prec == "fp64" else torch.float32
+    A = _csr(G).to_dense()
+    for a, b, v in ((3, 3, 0.7), (n - 1, n - 1, 0.7), (3, n - 1, -0.7), (n - 1, 3, -0.7)):
+        A[a, b] += v
+    # a row of d <= 500 terms summed in the row's precision: d roundings of at most |A| |x|
+    bound = 500 * (2.0 ** -52 if prec == "fp64" else 2.0 ** -23)
+    for width in (R, 3, R):  # another partition and its scratch between two calls
+        x = torch.randn((n, width), dtype=dt, device="cuda", generator=torch.Generator("cuda").manual_seed(width))
+        want = A @ x.double()
+        size = A.abs() @ x.double().abs()
+        assert float(((op(x).double() - want).abs() / size).max()) < bound

@@ -102,3 +102,34 @@ def test_apply_partitions(prec, weighted, own, R):
         want = A @ x.double()
         size = A.abs() @ x.double().abs()
         assert float(((op(x).double() - want).abs() / size).max()) < bound
+
+
+# long lists of added edges on the kernel-per-phase driver; bounds as above
+@pytest.mark.parametrize("prec,tol,bound", [("fp64", 1e-8, 1.5e-8), ("mixed", 1e-6, 2e-4)])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("R,m", [(1, 600), (5, 40), (16, 700), (64, 5), (64, 900)])
+def test_added_edges_residual(prec, tol, bound, weighted, R, m):
+    import torch
+    import polar_b200 as pg
+    G = _graph(weighted)
+    op = pg.Op(G)
+    rng = np.random.default_rng(m)
+    pairs = rng.permutation(N)[:2 * m].reshape(m, 2)
+    hub = int(np.argmax(np.diff(G._indptr_h)))
+    pairs = np.vstack([pairs, [[hub, k] for k in (7, 11, 13) if k != hub]])  # several at a heavy row
+    w = rng.uniform(0.2, 2.0, len(pairs))
+    for (a, b), we in zip(pairs, w):
+        op.add(int(a), int(b), float(we))
+    gen = torch.Generator("cuda").manual_seed(R)
+    W = torch.randn((N, R), dtype=torch.float64, device="cuda", generator=gen)
+    tau = np.array([0.0, 2.0])
+    X, _, _ = pg.msolve(op, W, tau, np.arange(N), tol, precision=prec)
+    A = _csr(G)
+    a, b = (torch.as_tensor(pairs[:, k], device="cuda") for k in (0, 1))
+    wd = torch.as_tensor(w, device="cuda")[:, None]
+    for j, t in enumerate(tau):
+        x = X[j].double()
+        r = W - (A @ x + t * x)
+        d = wd * (x[a] - x[b])
+        r.index_add_(0, a, d, alpha=-1.0).index_add_(0, b, d)
+        assert float((r.norm(dim=0) / W.norm(dim=0)).max()) < bound

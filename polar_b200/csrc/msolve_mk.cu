@@ -170,15 +170,6 @@ POLAR_D void step_length(const SolvePrm<T>& P, const double* dv) {
 #endif
 // Bytes of gathered rows in flight per lane: the gather batch is this many bytes over the
 // lane's share of a row (at least one neighbour).  Larger batches spill at 64 registers.
-#ifndef POLAR_STREAM_U
-#define POLAR_STREAM_U 4  // row items in flight per thread in the d update
-#endif
-#ifndef POLAR_RESID_U
-#define POLAR_RESID_U 2   // same for the r update with FP64 vectors (more spills at 64 registers)
-#endif
-#ifndef POLAR_RESID_U32
-#define POLAR_RESID_U32 1  // same with FP32 v: one item at a time was 6 % faster at n = 4.0M, R = 16
-#endif
 #ifndef POLAR_STREAM_MINB
 #define POLAR_STREAM_MINB 2  // resident 512-thread CTAs per SM requested for the r and d updates
 #endif
@@ -400,6 +391,10 @@ __global__ void __launch_bounds__(kBlock) mk_added(const __grid_constant__ Solve
   }
 }
 
+// The r and d updates are bound by HBM (24 to 32 bytes per entry).  A thread takes one row item per
+// trip of its loop: the CTAs then walk the vectors side by side as one front, which DRAM serves
+// better than several items a grid apart (us per d update, two or four items -> one: n = 4.0M R = 16
+// mixed 255 -> 236, 6.5 TB/s; n = 317,000 R = 128 mixed 167 -> 157, R = 16 FP64 28.2 -> 25.2).
 // ---- r <- r - a v, history, r.r, column scalars -----------------------------------------
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kBlock, POLAR_STREAM_MINB) mk_resid(const __grid_constant__ SolvePrm<T> P, int slot) {
@@ -426,37 +421,24 @@ __global__ void __launch_bounds__(kBlock, POLAR_STREAM_MINB) mk_resid(const __gr
   }
   if (any_on) {
     T* hslot = P.hist + (size_t)slot * nA * ld;
-    constexpr int U = sizeof(T) == 4 ? POLAR_RESID_U32 : (VEC >= 4 && POLAR_RESID_U > 1 ? POLAR_RESID_U / 2 : POLAR_RESID_U);
-    for (long long e0 = tid; e0 < nvec; e0 += U * nth) {
-      double rv[U][VEC];
-      T vv[U][VEC];
-      long long ii[U];
-      int ai[U];
+    for (long long e = tid; e < nvec; e += nth) {
+      const long long i = e >> lgG;
+      const size_t o = (size_t)i * ld + rg.col;
+      double rv[VEC];
+      T vv[VEC], rt[VEC];
+      load_res<T, VEC>(P, rv, o);
+      vload<T, VEC, true>(vv, P.v + o);
+      const int ai = __ldg(P.active_pos + i);
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const long long e = e0 + u * nth;
-        ii[u] = e < nvec ? (e >> lgG) : -1;
-        if (ii[u] >= 0) {
-          load_res<T, VEC>(P, rv[u], (size_t)ii[u] * ld + rg.col);
-          vload<T, VEC, true>(vv[u], P.v + (size_t)ii[u] * ld + rg.col);
-          ai[u] = __ldg(P.active_pos + ii[u]);
-        }
+      for (int v = 0; v < VEC; ++v)
+        if (on[v]) rv[v] = rv[v] - a_c[v] * (double)vv[v];
+      store_res<T, VEC>(P, rv, o);
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) {
+        racc[v] += rv[v] * rv[v];
+        rt[v] = (T)rv[v];
       }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (ii[u] < 0) continue;
-        T rt[VEC];
-#pragma unroll
-        for (int v = 0; v < VEC; ++v)
-          if (on[v]) rv[u][v] = rv[u][v] - a_c[v] * (double)vv[u][v];
-        store_res<T, VEC>(P, rv[u], (size_t)ii[u] * ld + rg.col);
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) {
-          racc[v] += rv[u][v] * rv[u][v];
-          rt[v] = (T)rv[u][v];
-        }
-        if (ai[u] >= 0) vstore_cs<T, VEC, true>(hslot + (size_t)ai[u] * ld + rg.col, rt);
-      }
+      if (ai >= 0) vstore_cs<T, VEC, true>(hslot + (size_t)ai * ld + rg.col, rt);
     }
   }
   reduce_cols_to_part<VEC>(racc, rg.G, ld, red, P.part + (size_t)blockIdx.x * ld);
@@ -508,29 +490,16 @@ __global__ void __launch_bounds__(kBlock, POLAR_STREAM_MINB) mk_dir(const __grid
     if (any_on) {
       const uint64_t pol_hot = l2_policy(P.l2_mode ? 1 : 0);
       const uint64_t pol_norm = l2_policy(0);
-      // four FP64 columns take the registers of two row items of two
-      constexpr int U = (VEC >= 4 && POLAR_STREAM_U > 2) ? 2 : POLAR_STREAM_U;
-      for (long long e0 = tid; e0 < nvec; e0 += U * nth) {
-        double rv[U][VEC], dv[U][VEC];
-        long long ii[U];
+      for (long long e = tid; e < nvec; e += nth) {
+        const long long i = e >> lgG;
+        const size_t o = (size_t)i * ld + rg.col;
+        double rv[VEC], dv[VEC];
+        load_res<T, VEC>(P, rv, o);
+        load_dir<T, VEC>(P, dv, o);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const long long e = e0 + u * nth;
-          ii[u] = e < nvec ? (e >> lgG) : -1;
-          if (ii[u] >= 0) {
-            load_res<T, VEC>(P, rv[u], (size_t)ii[u] * ld + rg.col);
-            load_dir<T, VEC>(P, dv[u], (size_t)ii[u] * ld + rg.col);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (ii[u] < 0) continue;
-#pragma unroll
-          for (int v = 0; v < VEC; ++v)
-            if (on[v]) dv[u][v] = rv[u][v] + be_c[v] * dv[u][v];
-          store_dir_hint<T, VEC>(P, dv[u], (size_t)ii[u] * ld + rg.col, row_policy(P, ii[u], pol_hot, pol_norm),
-                                 pol_norm);
-        }
+        for (int v = 0; v < VEC; ++v)
+          if (on[v]) dv[v] = rv[v] + be_c[v] * dv[v];
+        store_dir_hint<T, VEC>(P, dv, o, row_policy(P, i, pol_hot, pol_norm), pol_norm);
       }
     }
   }

@@ -62,7 +62,10 @@ POLAR_D unsigned cl_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+// Barrier of the cluster's threads.  The aligned forms need every lane of a warp at the same
+// instruction, so the warp joins up here: callers arrive from one-lane branches.
 POLAR_D void cl_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -102,7 +105,6 @@ POLAR_D void cl_exchange(ClShared<T, CG>& S, int which, int cs, int rank) {
     if (cs == 1) S.xbuf[which][0][c] = v[0];
     else cl_store(&S.xbuf[which][rank][c], dst, v[0]);
   }
-  __syncwarp();
   if (cs == 1) __syncthreads();
   else cl_sync();
 }
@@ -742,7 +744,6 @@ POLAR_D void cl_run(const SolvePrm<T>& P, const int grp) {
         }
       }
     }
-    __syncwarp();
     if (cs > 1) {  // barrier 3
       cl_sync();
       if (more) collect();

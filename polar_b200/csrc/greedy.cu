@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(kMaintBlock, NT <= 2 ? 3 : 1) maint_rows_kerne
   constexpr int LPR = 8;
   const int j = blockIdx.y, lg = threadIdx.x & (LPR - 1);
   const int uc = win[0];
-  const double D = m.D[j], rD = 1.0 / D;
+  const double D = m.D[j];
   double xi[NT][VEC], eta[NT][VEC];
 #pragma unroll
   for (int k = 0; k < NT; ++k)
@@ -391,8 +391,7 @@ __global__ void __launch_bounds__(kMaintBlock, NT <= 2 ? 3 : 1) maint_rows_kerne
         }
       }
       u = ldv(U, u_f32, ((size_t)j * nA + a) * ldu + uc);
-      const double q0 = u * rD;
-      const double ud = fma(fma(-q0, D, u), rD, q0);  // u / D
+      const double ud = u / D;
 #pragma unroll
       for (int k = 0; k < NT; ++k) {
         const int c = c0 + (k * LPR + lg) * VEC;

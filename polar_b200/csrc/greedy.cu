@@ -348,12 +348,12 @@ __global__ void maint_setup_kernel(const void* X, int ldx, const void* Y, int ld
 }
 
 // w = row . dir (before the update), then X_row -= u xi / D, Y_row += u eta / D, for the rows of
-// one pole (blockIdx.y): 8 lanes per row, each with NT x VEC of its columns, whose xi and eta
+// one pole: 8 lanes per row, each with NT x VEC of its columns, whose xi and eta
 // stay in registers over the CTA's rows (reading them again for every row was 2 KB from L1 for
 // the row's own 512 bytes: 2,210 us at 24 x 226,000 rows, q = 64 mixed; 1,050 us now, the
 // bytes of X and Y being 850).
 constexpr int kMaintBlock = 256;
-constexpr int kMaintRows = 512;  // rows per CTA
+constexpr int kMaintRows = 512;  // rows per CTA: CTAs of pole 0, then of pole 1, ... (poles are not bounded)
 
 template <typename T, int VEC, int NT>
 __global__ void __launch_bounds__(kMaintBlock, NT <= 2 ? 3 : 1) maint_rows_kernel(T* X, int ldx, T* Y, int ldy, int nA, int q, int c0,
@@ -361,7 +361,8 @@ __global__ void __launch_bounds__(kMaintBlock, NT <= 2 ? 3 : 1) maint_rows_kerne
                                                                  const int32_t* win, MaintTmp m) {
   // columns [c0, c1) of q (a wide bank goes in several launches, whose dots add up)
   constexpr int LPR = 8;
-  const int j = blockIdx.y, lg = threadIdx.x & (LPR - 1);
+  const int nb = (nA + kMaintRows - 1) / kMaintRows;
+  const int j = blockIdx.x / nb, lg = threadIdx.x & (LPR - 1);
   const int uc = win[0];
   const double D = m.D[j];
   double xi[NT][VEC], eta[NT][VEC];
@@ -373,8 +374,8 @@ __global__ void __launch_bounds__(kMaintBlock, NT <= 2 ? 3 : 1) maint_rows_kerne
       xi[k][v] = c < c1 ? m.xi[(size_t)j * q + c] : 0.0;
       eta[k][v] = c < c1 ? m.eta[(size_t)j * q + c] : 0.0;
     }
-  const int a1 = min(nA, (int)(blockIdx.x + 1) * kMaintRows);
-  for (int a0 = blockIdx.x * kMaintRows; a0 < a1; a0 += kMaintBlock / LPR) {
+  const int first = (blockIdx.x - j * nb) * kMaintRows, a1 = min(nA, first + kMaintRows);
+  for (int a0 = first; a0 < a1; a0 += kMaintBlock / LPR) {
     const int a = a0 + threadIdx.x / LPR;
     const bool ok = a < a1;
     T xv[NT][VEC], yv[NT][VEC];
@@ -585,7 +586,7 @@ static int maintain(void* d_X, int ldx, void* d_Y, int ldy, int xy_f32, int p, i
   int rc = check_launch("maint_setup");
   if (rc) return rc;
   const uintptr_t al = (uintptr_t)d_X | (uintptr_t)d_Y;
-  const dim3 grid((nA + kMaintRows - 1) / kMaintRows, p);
+  const int ctas = (nA + kMaintRows - 1) / kMaintRows * p;
   auto rows = [&](auto* x, auto* y, auto vec) {
     using T = std::remove_pointer_t<decltype(x)>;
     constexpr int V = decltype(vec)::value;
@@ -593,7 +594,7 @@ static int maintain(void* d_X, int ldx, void* d_Y, int ldy, int xy_f32, int p, i
       const int c1 = q - c0 < 8 * 8 * V ? q : c0 + 8 * 8 * V;
       const int trips = (c1 - c0 + 8 * V - 1) / (8 * V);
       auto go = [&](auto nt) {
-        maint_rows_kernel<T, V, decltype(nt)::value><<<grid, kMaintBlock, 0, st>>>(x, ldx, y, ldy, nA, q, c0, c1, d_U,
+        maint_rows_kernel<T, V, decltype(nt)::value><<<ctas, kMaintBlock, 0, st>>>(x, ldx, y, ldy, nA, q, c0, c1, d_U,
                                                                                    u_f32, ldu, d_win, m);
       };
       if (trips <= 1) go(std::integral_constant<int, 1>{});

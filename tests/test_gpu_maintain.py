@@ -58,3 +58,22 @@ def test_update_divides_by_any_denominator(prec, ua, ub):
                 np.testing.assert_array_equal(got[big], want.astype(dt)[big])
                 err = np.abs(got.astype(np.float64) - want)[~big] / size[~big]
                 assert err.size == 0 or err.max() < (2.0 ** -22 if prec == "mixed" else 2.0 ** -50)
+
+
+def test_more_poles_than_a_grid_dimension():
+    p, nA, q = 65537, 3, 2
+    rng = np.random.default_rng(1)
+    X, Y = rng.normal(size=(2, p, nA, q))
+    U = rng.uniform(-0.2, 0.2, (p, nA, 1))
+    G = rng.normal(size=(1, q))
+    h, t = rng.uniform(0.0, 1.0, (2, p, 1))
+    Xn, Yn, hn, tn = _maintain(X, Y, U, _win(0, 0, 2, 0), G, np.array([[1, 2]], np.int32), h, t)
+    u = U[:, :, 0]
+    xi, eta = X[:, 0] - X[:, 2], G - (Y[:, 0] - Y[:, 2])
+    ud = u / (1.0 + u[:, :1] - u[:, 2:])
+    cc = ud[:, 1] - ud[:, 2]
+    for got, want in ((Xn, X - ud[:, :, None] * xi[:, None]), (Yn, Y + ud[:, :, None] * eta[:, None]),
+                      (hn[:, 0], np.maximum(0, h[:, 0] - 2 * cc * ((X[:, 1] - X[:, 2]) * xi).sum(1) + cc * cc * (xi * xi).sum(1))),
+                      (tn[:, 0], np.maximum(0, t[:, 0] + 2 * cc * ((Y[:, 1] - Y[:, 2]) * eta).sum(1) + cc * cc * (eta * eta).sum(1)))):
+        # a dozen roundings of terms of at most a few hundred
+        np.testing.assert_allclose(got, want, rtol=1e-12, atol=1e-12)

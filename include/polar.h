@@ -175,9 +175,16 @@ int polar_msolve_finish(void* d_workspace, polar_stream_t stream, polar_msolve_i
 void polar_set_barrier_timeout_ns(uint64_t ns);
 /* Solver driver: 0 (default) one high-occupancy kernel per phase, M iterations per
  * CUDA-graph launch, host checks convergence once per launch (polar_msolve then returns
- * after the solve), or, for graphs whose direction fits an SM's shared memory, the whole
- * solve in one launch of a kernel per column group (thread-block clusters); 1: one persistent cooperative kernel with bounded grid barriers. */
+ * after the solve), or, for graphs whose direction fits an SM's shared memory, the cluster
+ * solver: the whole solve in one launch, a thread-block cluster per column group (where its
+ * estimated time is the shorter one); 1: one persistent cooperative kernel with bounded grid
+ * barriers. */
 int polar_set_solver_mode(int mode);
+/* 0: polar_msolve calls of this host thread with driver 0 take the kernels per phase on every
+ * graph; 1 (default): the cluster solver where it is estimated to be faster.  Returns the
+ * thread's previous setting.  The layout and cache settings below (lane bytes, sliced ELL, L2
+ * policy) concern the kernels per phase only. */
+int polar_set_cluster_solver(int on);
 /* Degree above which polar_msolve expects a row to be chunked for an R-column solve in
  * this precision: 8 x (lanes per row).  Heavy rows are split into chunks of at most 256
  * neighbours (polar_graph h_* fields), each processed by one warp. */

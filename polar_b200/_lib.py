@@ -94,6 +94,7 @@ SIGNATURES = {
     "polar_msolve_finish": (_I, [_P, _P, ctypes.POINTER(MsolveInfo)]),
     "polar_set_barrier_timeout_ns": (None, [ctypes.c_uint64]),
     "polar_set_solver_mode": (_I, [_I]),
+    "polar_set_cluster_solver": (_I, [_I]),
     "polar_heavy_threshold": (_I, [_I, _I]),
     "polar_sell_rows": (_I, [_I, _I]),
     "polar_set_spmm_lane_bytes": (None, [_I]),

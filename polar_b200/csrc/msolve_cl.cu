@@ -1031,6 +1031,9 @@ struct ClResident {
   }
 };
 
+// Whether this thread's solves may take the cluster kernel.
+thread_local bool g_cluster = true;
+
 int cl_resident(int cs) {
   static const ClResident r;
   return r.most[cs];
@@ -1145,7 +1148,7 @@ size_t cl_graph_layout(const polar_graph* g, int nA, char* base, ClGraph* C) {
 // columns the cluster solver is the faster one wherever the direction fits, by up to 2.9x.
 template <typename T>
 bool cl_fits(const SolvePrm<T>& P) {
-  if (P.r32 || !P.cl.head) return false;
+  if (!g_cluster || P.r32 || !P.cl.head) return false;
   const double bytes = (double)P.ld * sizeof(T);
   const double other = 85000 + bytes * (0.0076 * P.g.n + 0.00011 * P.g.nnz + 2e-5 * (4.0 * P.p + kHist) * P.nA);
   return cl_plan(P).cost < other;
@@ -1202,3 +1205,9 @@ template int cl_solve_one<float>(const SolvePrm<float>&, cudaStream_t, MkResult*
 template int cl_solve_one<double>(const SolvePrm<double>&, cudaStream_t, MkResult*);
 
 }  // namespace polar
+
+extern "C" int polar_set_cluster_solver(int on) {
+  const int was = polar::g_cluster ? 1 : 0;
+  polar::g_cluster = on != 0;
+  return was;
+}

@@ -14,7 +14,8 @@ import torch
 
 from . import _lib
 
-__all__ = ["msolve", "Counter", "precision_code", "max_columns", "prepare_active", "set_solver_mode"]
+__all__ = ["msolve", "Counter", "precision_code", "max_columns", "prepare_active", "set_solver_mode",
+           "set_cluster_solver"]
 
 
 def set_solver_mode(mode):
@@ -22,6 +23,12 @@ def set_solver_mode(mode):
     'persistent': a single cooperative kernel with bounded grid barriers."""
     code = {"graph": 0, "persistent": 1}[mode]
     _lib.check(_lib.load().polar_set_solver_mode(code), "set_solver_mode")
+
+
+def set_cluster_solver(on):
+    """Whether this thread's msolve calls with the 'graph' driver may take the cluster solver
+    (a small graph's whole solve in one launch; default True).  Returns the previous setting."""
+    return bool(_lib.load().polar_set_cluster_solver(1 if on else 0))
 
 
 class Counter:

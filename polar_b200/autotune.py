@@ -9,11 +9,14 @@ warp per row, 32 columns per pass).  Here the multi-shift CG's SpMM has three kn
 * the sliced-ELL copy of the light rows (on: warps read the neighbour lists of their rows
   slice-wise; off: CSR row loop);
 * the heavy-row threshold, as a multiple (4, 8, 16, 32 or 128) of the lanes per row: rows
-  above it are cut into chunks of at most 256 neighbours, one warp each.
+  above it are cut into the chunks of solver.heavy_partition (64, 128 or 256 neighbours by
+  graph size), one warp each.
 
 tune_msolve times `iters` iterations of the real solver (kernel-per-phase driver, CUDA
 graph blocks) for every combination and records the fastest; msolve then applies the
-recorded choice (kept on the Graph object) whenever it solves that graph at that width.  Results are identical up to
+recorded choice (kept on the Graph object) whenever it solves that graph at that width with
+that driver.  Solves that the cluster solver takes have no such layout; tuning leaves it aside,
+or every layout would time the same kernel.  Results are identical up to
 summation order (the heavy split changes which partial sums are formed).
 """
 import time
@@ -82,6 +85,7 @@ def tune_msolve(op, R, precision="mixed", p=8, iters=64, reps=2, lane_bytes=LANE
     saved = reg.pop(key, None)
     table = []
     seen = set()
+    cluster = _solver.set_cluster_solver(False)
     try:
         for lb in lane_bytes:
             lanes = _lanes(prec, ld, lb)
@@ -109,6 +113,7 @@ def tune_msolve(op, R, precision="mixed", p=8, iters=64, reps=2, lane_bytes=LANE
                         best = dt if best is None else min(best, dt)
                     table.append((lb, sell, thresh, best))
     finally:
+        _solver.set_cluster_solver(cluster)
         reg.pop(key, None)
         if saved is not None:
             reg[key] = saved

@@ -131,3 +131,20 @@ def test_setting_belongs_to_the_thread():
         assert got == [True]
     finally:
         assert solver.set_cluster_solver(True) is False
+
+
+@pytest.mark.parametrize("prec,R", [("fp64", 16), ("mixed", 64)])
+def test_tuner_times_the_kernels_per_phase(prec, R):
+    import polar_b200 as pg
+    from polar_b200 import _lib, autotune, solver
+    lib = _lib.load()
+    op = pg.Op(pg.Graph(4000, chung_lu(4000, 8.0, 2.1, 21, min_degree=1), 1e-2))
+    lib.polar_set_kernel_timing(1)
+    try:
+        res = autotune.tune_msolve(op, R, prec, iters=16, reps=1, heavy_mult=(4, 32))
+        seen = {k: v[0] for k, v in _lib.kernel_timing().items()}
+    finally:
+        lib.polar_set_kernel_timing(0)
+    # two runs of 16 iterations per layout
+    assert seen["cluster"] == 0 and seen["resid"] == 32 * len(res["table"])
+    assert solver.set_cluster_solver(True) is True

@@ -254,6 +254,8 @@ class Graph:
             t, ch = self._fine_partition(0)
             if t < self.heavy_thresh:
                 self._heavy_parts(t, ch)
+        if self.weighted:  # the panel kernel's
+            self._row_blocks(hv)
 
     def _fine_partition(self, row_bytes):
         """(threshold, chunk) of an apply with rows of that many bytes."""
@@ -262,8 +264,9 @@ class Graph:
         return (64 if self.n < 1_000_000 else self.heavy_thresh), 128
 
     def _row_blocks(self, hv):
-        """Row blocks of a partition, built when a kernel first streams through them (the
-        sliced-ELL kernels do not; 10 ms on the host at n = 317,000)."""
+        """Row blocks of a partition.  Only the panel kernel and the persistent driver stream
+        through them: weighted graphs build their own partition's with the graph, others when
+        the sliced-ELL layout is switched off (host time: 10 ms at n = 317,000, 228 at 4.0M)."""
         if "nrb" not in hv:
             rb = row_blocks(self._indptr_h, hv["thresh"])
             hv.update(rowblk_h=rb, rowblk=_i32(rb.ravel() if len(rb) else np.zeros(2, np.int32), self.device),
@@ -465,7 +468,7 @@ class Op:
             return self.struct()
         thresh, chunk = self.G._fine_partition(R * (16 // vec))
         if self.G.heavy_thresh <= thresh:
-            return self.struct(sell_rows=sell)
+            return self.struct(sell_rows=sell, row_blocks=False)
         return self.struct(heavy_thresh=thresh, sell_rows=sell, chunk=chunk, row_blocks=False)
 
     def _scratch_for(self, lib, g, prec, maxc, stream):

@@ -1,9 +1,28 @@
 // Host-side CTA split of a batched persistent launch (no CUDA): kept in a header of its
 // own so that a plain C++ compiler can test it.
 #pragma once
+#include <algorithm>
 #include <vector>
 
 namespace polar {
+
+// Factor on the grids of solves that run side by side.  share[b]: problem b's rows, 1 for as many
+// as fill the GPU; its grid takes min(1, factor * share[b]) of it.  The factor is the largest up
+// to 1 with which the grids together ask for at most `most` GPUs, but at least `least`.
+inline double grid_factor(const std::vector<double>& share, double most, double least) {
+  auto asked = [&](double f) {
+    double s = 0.0;
+    for (double x : share) s += std::min(1.0, f * x);
+    return s;
+  };
+  if (asked(1.0) <= most) return 1.0;
+  double lo = least, hi = 1.0;
+  for (int k = 0; k < 60; ++k) {
+    const double mid = 0.5 * (lo + hi);
+    (asked(mid) <= most ? lo : hi) = mid;
+  }
+  return lo;
+}
 
 // CTA split: one CTA per problem, the rest in proportion to cost (largest remainders),
 // each problem capped where its row streams would give a thread fewer than two items.

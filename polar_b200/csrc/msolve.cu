@@ -813,7 +813,6 @@ static int batch_graph_run(const polar_msolve_problem* probs, int nprob, int ld,
                            cudaStream_t st) {
   std::vector<SolvePrm<T>> prm(nprob);
   std::vector<double> frac(nprob);
-  double shares = 0.0;
   const int full = mk_grid_max<T, VEC, W, E>();
   for (int b = 0; b < nprob; ++b) {
     const polar_msolve_problem& q = probs[b];
@@ -828,13 +827,12 @@ static int batch_graph_run(const polar_msolve_problem* probs, int nprob, int ld,
     prm[b].hot_rows /= nprob;  // concurrent solves share the L2
     // two row items per thread of the full grid count as a full share
     frac[b] = (double)q.g->n * (ld / VEC) / ((double)full * kBlock * 2.0);
-    shares += frac[b];
   }
   // Grids that together ask for much more than the GPU wait in each other's way: a kernel ends
   // with the CTA that was placed last.  They shrink until they ask for 2.5 GPUs, but not below
   // eight row items per thread (eight graphs of 5,000 to 60,000 rows, R = 64 mixed, items per
   // thread 2 / 4 / 8 / 16: 89 / 83 / 79 / 87 ms).
-  const double shrink = std::max(0.25, std::min(1.0, 2.5 / shares));
+  const double shrink = grid_factor(frac, 2.5, 0.25);
   for (double& f : frac) f = std::min(1.0, f * shrink);
   std::vector<MkResult> res;
   const int rc = mk_solve_batch<T, VEC, W, E>(prm, frac, st, res);

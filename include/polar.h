@@ -163,7 +163,9 @@ int polar_spmm_noalloc(const polar_graph* g, int precision, int R, double shift,
  * host loop stands in for the reference's host-side convergence check every 8 iterations,
  * polar_gpu.py:126).  It therefore cannot be captured into a caller's CUDA graph.  With
  * driver 1 the call returns after one cooperative launch.  In both cases
- * polar_msolve_finish synchronises the stream and returns the solve status. */
+ * polar_msolve_finish synchronises the stream and returns the solve status.
+ * Workspace: queried under the settings of the solve; more when the cluster solver takes it
+ * (polar_set_cluster_solver).  One that holds only the kernels per phase is solved by them. */
 size_t polar_msolve_workspace_bytes(const polar_graph* g, int precision, int R, int p, int nA);
 int polar_msolve(const polar_graph* g, int precision, const double* d_W, int ldw, int R,
                  const double* d_tau, int p, const int32_t* d_active, const int32_t* d_active_pos,

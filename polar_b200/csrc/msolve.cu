@@ -409,11 +409,13 @@ static char* ws_base(void* ws) { return (char*)align256((size_t)ws); }
 
 static int max_grid_for(int precision, int vec, bool weighted);
 
-static void solve_layout(const polar_graph* g, int precision, int R, int p, int nA, int grid, SolveLayout* L) {
+// cluster: with the regions of the cluster solver.
+static void solve_layout(const polar_graph* g, int precision, int R, int p, int nA, int grid, bool cluster,
+                         SolveLayout* L) {
   const int ld = choose_ld(precision, R);
   const size_t ts = precision == POLAR_MIXED ? 4 : 8;
   // the cluster solver lays the row vectors out by places, a few more than rows
-  const size_t n = g->n <= kClMaxRows ? (size_t)g->n + kClPad : (size_t)g->n;
+  const size_t n = (size_t)g->n + (cluster ? kClPad : 0);
   size_t o = 0;
   int k = 0;
   auto add = [&](size_t bytes) {
@@ -425,8 +427,7 @@ static void solve_layout(const polar_graph* g, int precision, int R, int p, int 
   add(n * ld * ts);                                // 2 v
   add((size_t)kHist * nA * ld * ts);               // 3 hist
   add((size_t)p * nA * ld * ts);                   // 4 P
-  // 5 X (the cluster solver keeps it in FP64)
-  add((size_t)p * nA * ld * (g->n <= kClMaxRows ? 8 : ts));
+  add((size_t)p * nA * ld * (cluster ? 8 : ts));   // 5 X (the cluster solver keeps it in FP64)
   add((size_t)(g->nchunks > 0 ? g->nchunks : 1) * ld * 8);   // 6 chunk partials (FP64 sums)
   add((size_t)(g->nheavy > 0 ? g->nheavy : 1) * 4 * (ld > 16 ? ld / 16 : 1));  // 7 heavy counters per panel
   add((size_t)grid * ld * 8);                      // 8 CTA partials
@@ -444,7 +445,7 @@ static void solve_layout(const polar_graph* g, int precision, int R, int p, int 
   add((size_t)p * ld * kNC * 8);                   // 31 composed deferred-update coefficients
   add((size_t)kMaxHeavyCtas * ld * 8);             // 32 heavy-row d.v partials
   add(precision == POLAR_MIXED ? n * ld * 4 : 0);  // 33 direction remainder (mixed precision)
-  add(cl_graph_bytes(g, nA));                       // 34 cluster solver: row order and lists
+  add(cluster ? cl_graph_bytes(g, nA) : 0);        // 34 cluster solver: row order and lists
   L->total = o + kWsAlign;  // the regions start at the first aligned byte of the workspace
   L->ld = ld;
   L->vec = choose_vec(precision, ld);
@@ -559,22 +560,30 @@ extern "C" int polar_set_solver_mode(int mode) {
   return POLAR_OK;
 }
 
+// Whether a solve takes the cluster solver (its kernels hold r in FP64 only).
+static bool takes_cluster(const polar_graph* g, int precision, int R, int p, int nA) {
+  return g_solver_mode == 0 && !(precision == POLAR_MIXED && g_mixed_residual_bits == 32) &&
+         cl_takes(g, precision, R, choose_ld(precision, R), p, nA);
+}
+
 extern "C" size_t polar_msolve_workspace_bytes(const polar_graph* g, int precision, int R, int p, int nA) {
   if (!g || R < 1 || p < 1 || nA < 0) return 0;
   const int ld = choose_ld(precision, R);
   SolveLayout L;
-  solve_layout(g, precision, R, p, nA, grid_for_mode(precision, choose_vec(precision, ld), g->d_wts != nullptr), &L);
+  solve_layout(g, precision, R, p, nA, grid_for_mode(precision, choose_vec(precision, ld), g->d_wts != nullptr),
+               takes_cluster(g, precision, R, p, nA), &L);
   return L.total;
 }
 
 // Parameter block of one solve: arguments as polar_msolve takes them, workspace regions
 // from the layout.  `composed`: deferred updates from composed coefficients (the
-// kernel-per-phase driver); the persistent kernels apply the per-step coefficients.
+// kernel-per-phase driver); the persistent kernels apply the per-step coefficients.  `cluster`:
+// the layout has the cluster solver's regions.
 template <typename TT>
 static void fill_prm(SolvePrm<TT>& prm, const polar_graph* g, int R, int ld, int p, int nA, double tol,
                      int64_t maxit, int track, const double* d_W, int ldw, const double* d_tau,
                      const int32_t* d_active, const int32_t* d_active_pos, void* d_X_out, int x_f32, int ldx,
-                     double* d_h_out, int64_t* d_iters_out, char* ws, const SolveLayout& L, bool composed) {
+                     double* d_h_out, int64_t* d_iters_out, char* ws, const SolveLayout& L, bool composed, bool cluster) {
   prm.g = *g;
   prm.n = g->n;
   prm.R = R;
@@ -630,7 +639,7 @@ static void fill_prm(SolvePrm<TT>& prm, const polar_graph* g, int R, int ld, int
   prm.part_h = (double*)(ws + L.off[32]);
   prm.dlo = sizeof(TT) == 4 ? (float*)(ws + L.off[33]) : nullptr;
   prm.cl.head = nullptr;
-  if (composed && g->n <= kClMaxRows) {
+  if (cluster) {
     cl_graph_layout(g, nA, ws + L.off[34], &prm.cl);
     prm.cl.X = (double*)(ws + L.off[5]);
   }
@@ -659,7 +668,12 @@ extern "C" int polar_msolve(const polar_graph* g, int precision, const double* d
   const bool weighted = g->d_wts != nullptr;
   const int grid = grid_for_mode(precision, vec, weighted);
   SolveLayout L;
-  solve_layout(g, precision, R, p, nA, grid, &L);
+  bool cluster = takes_cluster(g, precision, R, p, nA);
+  solve_layout(g, precision, R, p, nA, grid, cluster, &L);
+  if (cluster && workspace_bytes < L.total) {  // sized under other settings: the kernels per phase need less
+    cluster = false;
+    solve_layout(g, precision, R, p, nA, grid, false, &L);
+  }
   if (workspace_bytes < L.total) return set_error(POLAR_ERR_WORKSPACE, "workspace too small");
   cudaStream_t st = (cudaStream_t)stream;
   char* ws = ws_base(d_workspace);
@@ -673,7 +687,7 @@ extern "C" int polar_msolve(const polar_graph* g, int precision, const double* d
 
   auto fill = [&](auto* prm_ptr) {
     fill_prm(*prm_ptr, g, R, ld, p, nA, tol, maxit, track, d_W, ldw, d_tau, d_active, d_active_pos, d_X_out, x_f32,
-             ldx, d_h_out, d_iters_out, ws, L, g_solver_mode == 0);
+             ldx, d_h_out, d_iters_out, ws, L, g_solver_mode == 0, cluster);
   };
   int rc;
   if (g_solver_mode == 0) {
@@ -682,7 +696,7 @@ extern "C" int polar_msolve(const polar_graph* g, int precision, const double* d
       SolvePrm<float> prm;
       fill(&prm);
       SolvePrm<float>* dp = (SolvePrm<float>*)(ws + L.off[30]);
-      if (cl_fits(prm)) rc = cl_solve_one(prm, st, &res);
+      if (cluster) rc = cl_solve_one(prm, st, &res);
       else if (vec == 4) rc = weighted ? mk_solve<float, 4, true, POLAR_E32>(prm, dp, st, &res) : mk_solve<float, 4, false, POLAR_E32>(prm, dp, st, &res);
       else if (vec == 2) rc = weighted ? mk_solve<float, 2, true, POLAR_E32>(prm, dp, st, &res) : mk_solve<float, 2, false, POLAR_E32>(prm, dp, st, &res);
       else rc = weighted ? mk_solve<float, 1, true, POLAR_E32>(prm, dp, st, &res) : mk_solve<float, 1, false, POLAR_E32>(prm, dp, st, &res);
@@ -690,7 +704,7 @@ extern "C" int polar_msolve(const polar_graph* g, int precision, const double* d
       SolvePrm<double> prm;
       fill(&prm);
       SolvePrm<double>* dp = (SolvePrm<double>*)(ws + L.off[30]);
-      if (cl_fits(prm)) rc = cl_solve_one(prm, st, &res);
+      if (cluster) rc = cl_solve_one(prm, st, &res);
       else if (vec == 2) rc = weighted ? mk_solve<double, 2, true, POLAR_E64>(prm, dp, st, &res) : mk_solve<double, 2, false, POLAR_E64>(prm, dp, st, &res);
       else rc = weighted ? mk_solve<double, 1, true, POLAR_E64>(prm, dp, st, &res) : mk_solve<double, 1, false, POLAR_E64>(prm, dp, st, &res);
     }
@@ -823,7 +837,7 @@ static int batch_graph_run(const polar_msolve_problem* probs, int nprob, int ld,
     if (e == cudaSuccess) e = cudaMemsetAsync(q.d_iters_out, 0, sizeof(int64_t) * q.R, st);
     if (e != cudaSuccess) return set_cuda_error("cudaMemsetAsync (batch)", e);
     fill_prm(prm[b], q.g, q.R, ld, q.p, q.nA, q.tol, q.maxit, q.track, q.d_W, q.ldw, q.d_tau, q.d_active,
-             q.d_active_pos, q.d_X_out, q.x_f32, q.ldx, q.d_h_out, q.d_iters_out, ws, L[b], true);
+             q.d_active_pos, q.d_X_out, q.x_f32, q.ldx, q.d_h_out, q.d_iters_out, ws, L[b], true, false);
     prm[b].hot_rows /= nprob;  // concurrent solves share the L2
     // two row items per thread of the full grid count as a full share
     frac[b] = (double)q.g->n * (ld / VEC) / ((double)full * kBlock * 2.0);
@@ -869,7 +883,7 @@ extern "C" size_t polar_msolve_batch_workspace_bytes(const polar_graph* g, int p
   const int ld = choose_ld(precision, R);
   SolveLayout L;
   solve_layout(g, precision, R, p, nA, batch_layout_grid(precision, choose_vec(precision, ld), g->d_wts != nullptr),
-               &L);
+               false, &L);
   return L.total;
 }
 
@@ -902,7 +916,7 @@ extern "C" int polar_msolve_batch(const polar_msolve_problem* probs, int nprob, 
   std::vector<int> cap(nprob), ctas;
   for (int b = 0; b < nprob; ++b) {
     const polar_msolve_problem& q = probs[b];
-    solve_layout(q.g, precision, q.R, q.p, q.nA, gmax, &L[b]);
+    solve_layout(q.g, precision, q.R, q.p, q.nA, gmax, false, &L[b]);
     if (q.workspace_bytes < L[b].total) return set_error(POLAR_ERR_WORKSPACE, "workspace too small (batch problem)");
     const double n = q.g->n, nnz = q.g->nnz;
     cost[b] = q.cost > 0.0 ? q.cost : (nnz + 2.0 * n) * ld / sqrt(q.g->sigma > 0.0 ? q.g->sigma : 1.0);
@@ -938,12 +952,12 @@ extern "C" int polar_msolve_batch(const polar_msolve_problem* probs, int nprob, 
     if (precision == POLAR_MIXED) {
       SolvePrm<float> prm;
       fill_prm(prm, q.g, q.R, ld, q.p, q.nA, q.tol, q.maxit, q.track, q.d_W, q.ldw, q.d_tau, q.d_active,
-               q.d_active_pos, q.d_X_out, q.x_f32, q.ldx, q.d_h_out, q.d_iters_out, ws, L[b], false);
+               q.d_active_pos, q.d_X_out, q.x_f32, q.ldx, q.d_h_out, q.d_iters_out, ws, L[b], false, false);
       e = cudaMemcpyAsync(ws + L[b].off[30], &prm, sizeof(prm), cudaMemcpyHostToDevice, st);
     } else {
       SolvePrm<double> prm;
       fill_prm(prm, q.g, q.R, ld, q.p, q.nA, q.tol, q.maxit, q.track, q.d_W, q.ldw, q.d_tau, q.d_active,
-               q.d_active_pos, q.d_X_out, q.x_f32, q.ldx, q.d_h_out, q.d_iters_out, ws, L[b], false);
+               q.d_active_pos, q.d_X_out, q.x_f32, q.ldx, q.d_h_out, q.d_iters_out, ws, L[b], false, false);
       e = cudaMemcpyAsync(ws + L[b].off[30], &prm, sizeof(prm), cudaMemcpyHostToDevice, st);
     }
     if (e != cudaSuccess) return set_cuda_error("parameter block upload (batch)", e);

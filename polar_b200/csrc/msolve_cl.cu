@@ -1039,36 +1039,43 @@ int cl_resident(int cs) {
   return r.most[cs];
 }
 
+// What the choice of a launch shape depends on.
+struct ClShape {
+  int n, nnz;
+  bool weighted;
+  int R, ld, p, nA;
+};
+
 template <typename T, int CG>
-void cl_try(const SolvePrm<T>& P, int cs, ClPlan& best) {
+void cl_try(const ClShape& S, int cs, ClPlan& best) {
   ClPlan s;
   s.cg = CG;
   s.cs = cs;
-  s.groups = (P.R + CG - 1) / CG;
-  s.LS = ((P.g.n + cs - 1) / cs + 31) / 32 * 32;
+  s.groups = (S.R + CG - 1) / CG;
+  s.LS = ((S.n + cs - 1) / cs + 31) / 32 * 32;
   const int most = cl_resident(cs);
-  if (most < 1 || (long long)cs * s.LS + 1 > 65536 || (long long)cs * s.LS > P.g.n + kClPad) return;
-  s.own = cl_smem<T, CG>(cs, s.LS, P.p, true) <= kClSmemMax;
-  s.smem = cl_smem<T, CG>(cs, s.LS, P.p, s.own);
+  if (most < 1 || (long long)cs * s.LS + 1 > 65536 || (long long)cs * s.LS > S.n + kClPad) return;
+  s.own = cl_smem<T, CG>(cs, s.LS, S.p, true) <= kClSmemMax;
+  s.smem = cl_smem<T, CG>(cs, s.LS, S.p, s.own);
   if (s.smem > kClSmemMax) return;
   // Clocks per iteration, fitted to solves of 2,000 to 57,000 rows with 4 to 18 neighbours: fixed
   // reductions and scalars; gathers; the CTA's rows, dearer when their vectors come from L2;
   // the deferred update; with several CTAs their barriers and the direction's exchange.
-  const double rows = (double)P.g.n / cs;
-  double c = 5000 + (0.25 + 0.02 * CG * sizeof(T) + (P.g.d_wts ? 0.3 : 0.0)) * P.g.nnz / cs + rows * CG * (s.own ? 3.0 : 4.5) +
-             0.015 * sizeof(T) * CG * (double)P.nA * P.p / cs;
-  if (cs > 1) c += 4000 + (double)P.g.n * CG * sizeof(T) / 30.0;
+  const double rows = (double)S.n / cs;
+  double c = 5000 + (0.25 + 0.02 * CG * sizeof(T) + (S.weighted ? 0.3 : 0.0)) * S.nnz / cs + rows * CG * (s.own ? 3.0 : 4.5) +
+             0.015 * sizeof(T) * CG * (double)S.nA * S.p / cs;
+  if (cs > 1) c += 4000 + (double)S.n * CG * sizeof(T) / 30.0;
   s.cost = c * std::max(1.0, std::ceil((double)s.groups / most));
   if (s.cost < best.cost) best = s;
 }
 
 template <typename T>
-ClPlan cl_plan(const SolvePrm<T>& P) {
+ClPlan cl_plan(const ClShape& S) {
   ClPlan best;
   for (int cs = 1; cs <= kClMaxCta; ++cs) {
-    cl_try<T, 1>(P, cs, best);
-    if (P.ld >= 2) cl_try<T, 2>(P, cs, best);
-    if (sizeof(T) == 4 && P.ld >= 4) cl_try<T, 4>(P, cs, best);
+    cl_try<T, 1>(S, cs, best);
+    if (S.ld >= 2) cl_try<T, 2>(S, cs, best);
+    if (sizeof(T) == 4 && S.ld >= 4) cl_try<T, 4>(S, cs, best);
   }
   return best;
 }
@@ -1107,7 +1114,6 @@ cudaError_t cl_launch(const SolvePrm<T>& P, const ClPlan& s, cudaStream_t st) {
 }  // namespace
 
 size_t cl_graph_bytes(const polar_graph* g, int nA) {
-  if (g->n > kClMaxRows) return 0;
   ClGraph C;
   return cl_graph_layout(g, nA, nullptr, &C);
 }
@@ -1147,17 +1153,22 @@ size_t cl_graph_layout(const polar_graph* g, int nA, char* base, ClGraph* C) {
 // iteration against 98 here; n = 28,200, 18 neighbours: 115 against 142); with fewer
 // columns the cluster solver is the faster one wherever the direction fits, by up to 2.9x.
 template <typename T>
-bool cl_fits(const SolvePrm<T>& P) {
-  if (!g_cluster || P.r32 || !P.cl.head) return false;
-  const double bytes = (double)P.ld * sizeof(T);
-  const double other = 85000 + bytes * (0.0076 * P.g.n + 0.00011 * P.g.nnz + 2e-5 * (4.0 * P.p + kHist) * P.nA);
-  return cl_plan(P).cost < other;
+static bool cl_faster(const ClShape& S) {
+  const double bytes = (double)S.ld * sizeof(T);
+  const double other = 85000 + bytes * (0.0076 * S.n + 0.00011 * S.nnz + 2e-5 * (4.0 * S.p + kHist) * S.nA);
+  return cl_plan<T>(S).cost < other;
+}
+
+bool cl_takes(const polar_graph* g, int precision, int R, int ld, int p, int nA) {
+  if (!g_cluster || g->n > kClMaxRows) return false;
+  const ClShape S{g->n, g->nnz, g->d_wts != nullptr, R, ld, p, nA};
+  return precision == POLAR_MIXED ? cl_faster<float>(S) : cl_faster<double>(S);
 }
 
 template <typename T>
 int cl_solve_one(const SolvePrm<T>& P0, cudaStream_t st, MkResult* out) {
   SolvePrm<T> P = P0;
-  const ClPlan s = cl_plan(P);
+  const ClPlan s = cl_plan<T>(ClShape{P.g.n, P.g.nnz, P.g.d_wts != nullptr, P.R, P.ld, P.p, P.nA});
   P.cl.cs = s.cs;
   P.cl.LS = s.LS;
   P.cl.SL = s.LS + 2;
@@ -1199,8 +1210,6 @@ int cl_solve_one(const SolvePrm<T>& P0, cudaStream_t st, MkResult* out) {
   return POLAR_OK;
 }
 
-template bool cl_fits<float>(const SolvePrm<float>&);
-template bool cl_fits<double>(const SolvePrm<double>&);
 template int cl_solve_one<float>(const SolvePrm<float>&, cudaStream_t, MkResult*);
 template int cl_solve_one<double>(const SolvePrm<double>&, cudaStream_t, MkResult*);
 

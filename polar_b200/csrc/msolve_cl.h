@@ -7,14 +7,14 @@
 
 namespace polar {
 
-// Bytes of the graph's row order, places and neighbour lists for a cluster solve (0: graph too
-// large), and their pointers inside the workspace.
+// Bytes of the graph's row order, places and neighbour lists for a cluster solve, and their
+// pointers inside the workspace.
 size_t cl_graph_bytes(const polar_graph* g, int nA);
 size_t cl_graph_layout(const polar_graph* g, int nA, char* base, ClGraph* C);
 
-// True when the solve is taken by the cluster kernel.
-template <typename T>
-bool cl_fits(const SolvePrm<T>& P);
+// True when the cluster kernel is the faster one for a solve of this shape (ld: the padded R)
+// and this thread may take it.
+bool cl_takes(const polar_graph* g, int precision, int R, int ld, int p, int nA);
 
 // Runs a whole solve (blocking).
 template <typename T>

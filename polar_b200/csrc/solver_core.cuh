@@ -20,7 +20,7 @@ constexpr int kMaxHeavyCtas = 1024;    // bound of the heavy-row launch (partial
 #endif
 
 // Row order of the cluster solver (msolve_cl.cu): a row's place is CTA * LS + slot.
-constexpr int kClMaxRows = 60000;  // rows up to which a workspace carries it
+constexpr int kClMaxRows = 60000;  // rows up to which it is considered
 constexpr int kClPad = 4096;       // places and list entries beyond the rows' own
 
 struct ClGraph {
@@ -83,7 +83,7 @@ template <typename T> struct SolvePrm {
   // data evict_first, 2: cold gathers evict_first as well.
   int hot_rows;
   int l2_mode;
-  ClGraph cl;  // cluster solver (head == nullptr: not for this workspace)
+  ClGraph cl;  // cluster solver (head == nullptr: another driver's solve)
 };
 
 // Policy for a gather or store of row i of d.

@@ -24,8 +24,8 @@
 //
 // Layout.  cl_order sorts the rows by degree, deals them round the cluster's CTAs and numbers
 // every row by its place (CTA, slot).  A warp takes slices of 32 rows of up to kClLight
-// neighbours (a lane each), 4 rows of up to kClMid (8 lanes each) or one of up to kClWide, which
-// bounds its chain of gathers; a wider row takes the whole CTA.  cl_fill writes the
+// neighbours (a lane each), 4 rows of up to kClMid (8 lanes each) or one wider row, which bounds
+// its chain of gathers; a few very wide rows take the whole CTA (cl_order).  cl_fill writes the
 // neighbour lists in places, 16 bits each, as one stream of chunks per warp: a chunk is four
 // neighbours per lane (one 8-byte load), so that the next chunks are read ahead without
 // looking at the slices.
@@ -48,8 +48,8 @@ namespace {
 constexpr int kClMaxCta = 16;    // CTAs per cluster at most (non-portable size)
 constexpr int kClPoles = 16;     // poles per pass of the deferred update
 constexpr int kClLight = 16;     // neighbours up to which a row takes a lane,
-constexpr int kClMid = 256;      // 8 lanes
-constexpr int kClWide = 1024;    // and a warp; beyond, the whole CTA
+constexpr int kClMid = 256;      // 8 lanes; beyond, a warp
+constexpr int kClWide = 2048;    // neighbours above which a row may take the whole CTA
 constexpr int kClMidRows = 4;    // rows of a warp at 8 lanes each
 constexpr int kClAhead = 3;      // chunks past the end of a warp's neighbour stream that it may read
 constexpr int kItemD = 5 + kNC;  // doubles per (pole, column): z, zp, h, ip, pn, composed row
@@ -782,9 +782,12 @@ __global__ void __launch_bounds__(kBlock, 1) cl_solve(const __grid_constant__ So
 // ---- row order, places and neighbour lists of one problem -----------------------------------
 POLAR_D int cl_key(const polar_graph& g, int row) {
   const int deg = __ldg(g.d_indptr + row + 1) - __ldg(g.d_indptr + row);
-  // degree descending in classes that part kClLight, kClMid and kClWide: one per degree up to
-  // 64, then by 8 up to 512 and by 32 up to kClWide
-  const int c = deg <= 64 ? deg : deg <= 512 ? 64 + (deg - 57) / 8 : deg <= kClWide ? 121 + (deg - 481) / 32 : 255;
+  // degree descending in classes that part kClLight, kClMid and the powers of two from 1,024: one
+  // per degree up to 64, then by 8 up to 512, by 32 up to 1,024 and by doubling
+  const int c = deg <= 64     ? deg
+                : deg <= 512  ? 64 + (deg - 57) / 8
+                : deg <= 1024 ? 121 + (deg - 481) / 32
+                              : 128 + (31 - __clz(deg - 1));
   return 255 - c;
 }
 
@@ -819,6 +822,7 @@ POLAR_D int block_scan(int x, int* tmp, int* sum) {
 __global__ void __launch_bounds__(kOrderThreads) cl_order(polar_graph g, ClGraph C, const int* active_pos) {
   extern __shared__ int cnt[];  // 16 x kOrderThreads
   __shared__ int tmp[64];
+  __shared__ int over[5];  // rows of more than kClWide << k neighbours
   const int n = g.n, t = threadIdx.x;
   const int per = (n + kOrderThreads - 1) / kOrderThreads;
   const int lo = min(n, t * per), hi = min(n, lo + per);
@@ -856,15 +860,32 @@ __global__ void __launch_bounds__(kOrderThreads) cl_order(polar_graph g, ClGraph
     C.sx[i] = -1;
     C.sdiag[i] = 0.0;
   }
-  // rows above the limits of a warp, 8 lanes and one lane
-  int nv = 0, nh = 0, nm = 0;
+  // rows above the limits of 8 lanes and one lane
+  if (t < 5) over[t] = 0;
+  __syncthreads();
+  int nh = 0, nm = 0;
   for (int i = lo; i < hi; ++i) {
-    nv += degree(order[i]) > kClWide;
-    nh += degree(order[i]) > kClMid;
-    nm += degree(order[i]) > kClLight;
+    const int deg = degree(order[i]);
+    nh += deg > kClMid;
+    nm += deg > kClLight;
+    for (int k = 0; k < 5 && deg > kClWide << k; ++k) atomicAdd(&over[k], 1);
   }
-  int nwide, nhub, nmid;
-  block_scan(nv, tmp, &nwide);
+  __syncthreads();
+  // Rows of the whole CTA.  One costs all its warps two barriers and a serial sum, 1,500 clocks, and
+  // a clock per 14 neighbours; on a warp it is 0.7 clock per neighbour, the other warps having
+  // rows of their own.  So rows of more than L neighbours are taken by the CTA when its w of them
+  // are cheaper than one on a warp: from 4,096 when it has one, never from six on.  FP64 solves,
+  // rows of more than 1,024 on the CTA -> this: 2,500 rows of 1,100 neighbours R = 1 2.19 -> 0.98 ms;
+  // n = 20,000 with 50 rows of 5,000 R = 16 6.28 -> 5.14, with 300 of 1,200 7.51 -> 4.65.
+  int nwide = 0;
+  for (int k = 0; k < 5; ++k) {
+    const int L = kClWide << k, w = (over[k] + cs - 1) / cs;
+    if (w * (1500 + L / 14) < 0.7 * L) {
+      nwide = over[k];
+      break;
+    }
+  }
+  int nhub, nmid;
   block_scan(nh, tmp, &nhub);
   block_scan(nm, tmp, &nmid);
   __syncthreads();

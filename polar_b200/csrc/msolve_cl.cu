@@ -1062,7 +1062,7 @@ int cl_resident(int cs) {
 
 // What the choice of a launch shape depends on.
 struct ClShape {
-  int n, nnz;
+  int n, nnz, nx;
   bool weighted;
   int R, ld, p, nA;
 };
@@ -1079,9 +1079,10 @@ void cl_try(const ClShape& S, int cs, ClPlan& best) {
   s.own = cl_smem<T, CG>(cs, s.LS, S.p, true) <= kClSmemMax;
   s.smem = cl_smem<T, CG>(cs, s.LS, S.p, s.own);
   if (s.smem > kClSmemMax) return;
-  // Clocks per iteration, fitted to solves of 2,000 to 57,000 rows with 4 to 18 neighbours: fixed
-  // reductions and scalars; gathers; the CTA's rows, dearer when their vectors come from L2;
-  // the deferred update; with several CTAs their barriers and the direction's exchange.
+  // Clocks per iteration, for the choice between launch shapes, fitted to solves of 2,000 to 57,000
+  // rows with 4 to 18 neighbours: fixed reductions and scalars; gathers; the CTA's rows, dearer
+  // when their vectors come from L2; the deferred update; with several CTAs their barriers and
+  // the direction's exchange.
   const double rows = (double)S.n / cs;
   double c = 5000 + (0.25 + 0.02 * CG * sizeof(T) + (S.weighted ? 0.3 : 0.0)) * S.nnz / cs + rows * CG * (s.own ? 3.0 : 4.5) +
              0.015 * sizeof(T) * CG * (double)S.nA * S.p / cs;
@@ -1168,28 +1169,41 @@ size_t cl_graph_layout(const polar_graph* g, int nA, char* base, ClGraph* C) {
   return o;
 }
 
-// The other side of the choice is the kernel-per-phase driver's iteration: 45 us of launches,
-// reductions and gather latency, its vectors, gathers and deferred update (same solves, in
-// clocks).  At R = 128 the two meet near 30,000 rows (n = 29,800, 4 neighbours: 111 us an
-// iteration against 98 here; n = 28,200, 18 neighbours: 115 against 142); with fewer
-// columns the cluster solver is the faster one wherever the direction fits, by up to 2.9x.
+// Which driver is the faster one, from clocks per iteration of either, fitted (least squares of the
+// ratio) to 8,700 solves of 1,500 to 58,000 rows with 4 to 18 neighbours, 1 to 128 columns, half of
+// them with added edges.  Cluster: its fixed part (more with several CTAs), gathers, the CTA's
+// rows (dearer when their vectors come from L2), the deferred update, the direction's exchange,
+// added edges; as often as its clusters need turns.  Kernels per phase: launches, reductions and
+// gather latency, their vectors, and mk_added's launch or the SpMM's tail.  Of the solves 98.5 %
+// end up with the faster driver to 3 % (worst 1.36x); without terms for added edges 3 % of them
+// took the cluster solver though it was slower, by up to 1.7x (n = 28,000 R = 64 FP64 with 2,500
+// edges: 113 us an iteration, 82 by phases).
 template <typename T>
 static bool cl_faster(const ClShape& S) {
-  const double bytes = (double)S.ld * sizeof(T);
-  const double other = 85000 + bytes * (0.0076 * S.n + 0.00011 * S.nnz + 2e-5 * (4.0 * S.p + kHist) * S.nA);
-  return cl_plan<T>(S).cost < other;
+  const ClPlan b = cl_plan<T>(S);
+  if (b.groups == 0) return false;
+  const double rows = (double)S.n / b.cs, es = sizeof(T), own = b.own ? 1.7 : es == 8 ? 2.1 : 2.8;
+  double here = 6700 + (0.45 + (S.weighted ? 0.12 : 0.0)) * S.nnz / b.cs + rows * b.cg * own +
+                0.02 * es * b.cg * (double)S.nA * S.p / b.cs;
+  if (b.cs > 1) here += 6700 + 0.04 * es * b.cg * S.n;
+  if (S.nx > 0) here += 3200 + 20.0 * S.nx / b.cs;
+  here *= std::max(1.0, std::ceil((double)b.groups / cl_resident(b.cs)));
+  double phases = 75000 + 63 * es * S.ld + 0.018 * S.nnz + 0.02 * (double)S.ld * S.n;
+  if (S.weighted) phases += 11300 + 0.009 * S.nnz;
+  if (S.nx > 0) phases += added_split(S.nx, S.ld) ? 13000 + 0.04 * (double)S.nx * S.ld : 3300;
+  return here < phases;
 }
 
 bool cl_takes(const polar_graph* g, int precision, int R, int ld, int p, int nA) {
   if (!g_cluster || g->n > kClMaxRows) return false;
-  const ClShape S{g->n, g->nnz, g->d_wts != nullptr, R, ld, p, nA};
+  const ClShape S{g->n, g->nnz, g->nx, g->d_wts != nullptr, R, ld, p, nA};
   return precision == POLAR_MIXED ? cl_faster<float>(S) : cl_faster<double>(S);
 }
 
 template <typename T>
 int cl_solve_one(const SolvePrm<T>& P0, cudaStream_t st, MkResult* out) {
   SolvePrm<T> P = P0;
-  const ClPlan s = cl_plan<T>(ClShape{P.g.n, P.g.nnz, P.g.d_wts != nullptr, P.R, P.ld, P.p, P.nA});
+  const ClPlan s = cl_plan<T>(ClShape{P.g.n, P.g.nnz, P.g.nx, P.g.d_wts != nullptr, P.R, P.ld, P.p, P.nA});
   P.cl.cs = s.cs;
   P.cl.LS = s.LS;
   P.cl.SL = s.LS + 2;

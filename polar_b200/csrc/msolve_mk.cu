@@ -146,11 +146,9 @@ POLAR_D void apply_added_edges(const SolvePrm<T>& P, double* tmp, double* s_col)
   __syncthreads();
 }
 
-// Added edges go to mk_added when the SpMM's last CTA would need more than one pass of its
-// threads over the (row, column) items; up to that its tail is shorter than one more launch.
 template <typename T>
 POLAR_HD bool added_split(const SolvePrm<T>& P) {
-  return (long long)P.g.nx * P.ld > kBlock;
+  return added_split(P.g.nx, P.ld);
 }
 
 // a = rr / d.v per column, from the complete d.v (one CTA).

@@ -86,6 +86,10 @@ template <typename T> struct SolvePrm {
   ClGraph cl;  // cluster solver (head == nullptr: another driver's solve)
 };
 
+// Added edges go to mk_added when the SpMM's last CTA would need more than one pass of its
+// threads over the (row, column) items; up to that its tail is shorter than one more launch.
+POLAR_HD bool added_split(int nx, int ld) { return (long long)nx * ld > kBlock; }
+
 // Policy for a gather or store of row i of d.
 template <typename T>
 POLAR_D uint64_t row_policy(const SolvePrm<T>& P, long long i, uint64_t hot, uint64_t cold) {

@@ -86,3 +86,20 @@ def test_workspace_of_other_settings(prec, tol, bound, monkeypatch):
     with pytest.raises(_lib.PolarError) as e:
         pg.msolve(op, W, tau, act, tol, precision=prec)
     assert e.value.status == _lib.POLAR_ERR_WORKSPACE
+
+
+# shapes far from the line between the drivers: (n, nnz, rows with added edges, R, poles, active)
+@pytest.mark.parametrize("prec,shape,taken", [
+    ("fp64", (2000, 12000, 0, 1, 16, 2), True), ("fp64", (2000, 11000, 2000, 64, 16, 1000), True),
+    ("fp64", (20000, 110000, 6500, 16, 16, 1000), True), ("mixed", (20000, 110000, 6500, 128, 16, 1000), True),
+    ("fp64", (27647, 450000, 3929, 64, 15, 569), False), ("mixed", (50351, 463000, 2965, 48, 22, 3), False),
+    ("mixed", (50000, 274000, 7900, 64, 16, 1000), False), ("mixed", (50000, 1500000, 0, 64, 16, 1000), False),
+    ("fp64", (317000, 2000000, 0, 1, 16, 2), False)])
+def test_choice_between_drivers(prec, shape, taken):
+    from polar_b200 import _lib, solver
+    lib = _lib.load()
+    n, nnz, nx, R, p, nA = shape
+    g = _record(_lib, n, nnz)
+    g.nx = nx
+    ask = lambda: lib.polar_msolve_workspace_bytes(g, solver.precision_code(prec), R, p, nA)
+    assert (ask() > _phases(solver, ask)) == taken

@@ -312,11 +312,12 @@ extern "C" int polar_spmm(const polar_graph* g, int precision, int R, double shi
                        : try_spmm_sell<double>(*g, precision, R, shift, d_X, ldx, d_Y, ldy, d_scratch, st, &used);
     if (used || rs != POLAR_OK) return rs;
   }
-  const bool pow2 = (R & (R - 1)) == 0;
-  if (pow2 && ldx == R && precision == POLAR_MIXED && vec == 4)
+  // the panel kernel streams through row blocks; a graph without them takes the row loop
+  const bool panel = (R & (R - 1)) == 0 && g->d_rowblk != nullptr;
+  if (panel && ldx == R && precision == POLAR_MIXED && vec == 4)
     return w ? launch_spmm_panel<float, 4, true>(*g, R, shift, d_X, ldx, d_Y, ldy, d_scratch, st)
              : launch_spmm_panel<float, 4, false>(*g, R, shift, d_X, ldx, d_Y, ldy, d_scratch, st);
-  if (pow2 && ldx == R && precision == POLAR_FP64 && vec == 2)
+  if (panel && ldx == R && precision == POLAR_FP64 && vec == 2)
     return w ? launch_spmm_panel<double, 2, true>(*g, R, shift, d_X, ldx, d_Y, ldy, d_scratch, st)
              : launch_spmm_panel<double, 2, false>(*g, R, shift, d_X, ldx, d_Y, ldy, d_scratch, st);
   if (precision == POLAR_MIXED) {

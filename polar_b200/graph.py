@@ -314,6 +314,9 @@ class Graph:
         """Spectral upper bound sigma + 2 dmax + 4k (realworld/polar_gpu.py:59-60)."""
         return self.sigma + 2.0 * self.dmax + 4.0 * k
 
+    def _has_sell(self, thresh, S):
+        return (thresh, S) in getattr(self, "_sell_cache", ())
+
     def _sell(self, thresh, S):
         key = (thresh, S)
         if not hasattr(self, "_sell_cache"):
@@ -428,6 +431,10 @@ class _Added:
         s.d_xwt = self.wt_d.data_ptr() if self.wt_d is not None else None
 
 
+def _capturing(device):
+    return device.type == "cuda" and torch.cuda.is_current_stream_capturing()
+
+
 class Op:
     """y = (M0 + sum_S w b b^T + shift I) x  (realworld/polar_gpu.py:63-80)."""
 
@@ -467,20 +474,38 @@ class Op:
         if sell == 0 and whole and R & (R - 1) == 0:
             return self.struct()
         thresh, chunk = self.G._fine_partition(R * (16 // vec))
-        if self.G.heavy_thresh <= thresh:
+        own = self.G.heavy_thresh <= thresh
+        # nothing can be uploaded under stream capture: a layout that is not there yet is done without
+        if sell:
+            if not self.G._has_sell(self.G.heavy_thresh if own else thresh, sell) and _capturing(self.G.device):
+                sell = 0
+        elif not own and (thresh, chunk) not in self.G._heavy and _capturing(self.G.device):
+            own = True
+        if own:
             return self.struct(sell_rows=sell, row_blocks=False)
         return self.struct(heavy_thresh=thresh, sell_rows=sell, chunk=chunk, row_blocks=False)
 
-    def _scratch_for(self, lib, g, prec, maxc, stream):
+    def _prepare(self, lib, g, prec, maxc, stream):
         """Chunk partials and counters of `g`'s heavy-row partition: both their size and the
-        place of the counters follow from its numbers of chunks and rows."""
-        key = (prec, self.G.device.index, g.nchunks, g.nheavy)
-        if key not in self._scratch:
-            nb = lib.polar_spmm_scratch_bytes(g, prec, maxc)
+        place of the counters follow from its numbers of chunks and rows.  Where no width takes
+        the sliced-ELL layout, any can do with the graph's own partition: the first call prepares
+        that one too, and a call under stream capture takes it when its own is not there.
+        Returns the record to apply and its scratch."""
+        def key(x):
+            return prec, self.G.device.index, x.nchunks, x.nheavy
+        todo = [g]
+        if self.G.weighted or lib.polar_sell_rows(prec, maxc) == 0:
+            own = self.struct()
+            if key(own) not in self._scratch:
+                todo.append(own)
+            elif _capturing(self.G.device):
+                return own, self._scratch[key(own)]
+        for x in todo:
+            nb = lib.polar_spmm_scratch_bytes(x, prec, maxc)
             buf = torch.empty(max(nb, 256), dtype=torch.uint8, device=self.G.device)
-            _lib.check(lib.polar_spmm_scratch_init(g, prec, maxc, buf.data_ptr(), stream), "spmm scratch")
-            self._scratch[key] = buf
-        return self._scratch[key]
+            _lib.check(lib.polar_spmm_scratch_init(x, prec, maxc, buf.data_ptr(), stream), "spmm scratch")
+            self._scratch[key(x)] = buf
+        return g, self._scratch[key(g)]
 
     def __call__(self, x, shift=0.0):
         """Apply to an (n, R) or (n,) float64/float32 CUDA tensor; returns a new tensor."""
@@ -497,12 +522,15 @@ class Op:
         Y = torch.empty_like(X)
         lib = _lib.load()
         stream = torch.cuda.current_stream(X.device).cuda_stream
+        index = self.G.device.index
         for lo in range(0, R, maxc):
             hi = min(R, lo + maxc)
             xs = X[:, lo:hi]
             ys = Y[:, lo:hi]
             g = self._struct_for(lib, prec, hi - lo)
-            scratch = self._scratch_for(lib, g, prec, maxc, stream)
+            scratch = self._scratch.get((prec, index, g.nchunks, g.nheavy))
+            if scratch is None:
+                g, scratch = self._prepare(lib, g, prec, maxc, stream)
             _lib.check(lib.polar_spmm(g, prec, hi - lo, float(shift), xs.data_ptr(), R, ys.data_ptr(), R,
                                       scratch.data_ptr(), stream), "polar_spmm")
         return Y.reshape(-1) if squeeze else Y

@@ -17,8 +17,8 @@
 //
 // Why shared memory.  A random 8- or 16-byte gather costs an SM 1.7 clocks per lane through
 // L2 (one tag look-up per row, whatever its width) and 0.13 from its own shared memory, so
-// every CTA of a cluster holds the whole direction of its columns, n x CG values (up to 25,000
-// rows in FP64 and 50,000 in FP32 at CG = 1), and computes its share of the rows.  With more
+// every CTA of a cluster holds the whole direction of its columns, n x CG values (up to 28,000
+// rows in FP64 and 56,000 in FP32 at CG = 1), and computes its share of the rows.  With more
 // than one CTA the new direction goes through global memory once per iteration (own part
 // written, the others' read back, contiguous).
 //
@@ -1175,7 +1175,7 @@ size_t cl_graph_layout(const polar_graph* g, int nA, char* base, ClGraph* C) {
 // rows (dearer when their vectors come from L2), the deferred update, the direction's exchange,
 // added edges; as often as its clusters need turns.  Kernels per phase: launches, reductions and
 // gather latency, their vectors, and mk_added's launch or the SpMM's tail.  Of the solves 98.5 %
-// end up with the faster driver to 3 % (worst 1.36x); without terms for added edges 3 % of them
+// end up with the faster driver to 3 % (worst 1.27x); without terms for added edges 3 % of them
 // took the cluster solver though it was slower, by up to 1.7x (n = 28,000 R = 64 FP64 with 2,500
 // edges: 113 us an iteration, 82 by phases).
 template <typename T>

@@ -29,8 +29,9 @@ struct ClGraph {
   int *srow, *sact, *sx;  // place -> row, active row in place order, added-edge row (-1: none)
   double* sdiag;          // place -> diagonal without the shift
   int* aorig;             // active row in place order -> the caller's
-  int2* slice;            // per slice of a CTA: first list entry, pairs of places per lane
-  int* head;              // per CTA: rows of the CTA, a warp, 8 lanes; first active row, active rows
+  int2* slice;            // per slice of a CTA: first chunk, chunks (4 neighbours a lane each); a row of
+                          // the whole CTA: first list entry, neighbours
+  int* head;              // per CTA: rows of the CTA, a warp, 8 lanes; first active row, active rows; slices
   unsigned short* ell;    // neighbour lists in places
   double* ellw;           // and weights
   double* X;              // pole iterates, FP64 in both precisions

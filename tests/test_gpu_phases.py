@@ -148,3 +148,28 @@ def test_tuner_times_the_kernels_per_phase(prec, R):
     # two runs of 16 iterations per layout
     assert seen["cluster"] == 0 and seen["resid"] == 32 * len(res["table"])
     assert solver.set_cluster_solver(True) is True
+
+
+@pytest.mark.parametrize("prec,R", [("fp64", 1), ("fp64", 16), ("mixed", 16), ("mixed", 64)])
+def test_recorded_layouts_give_the_same_solve(prec, R):
+    """Lane bytes, sliced-ELL or CSR rows and the heavy-row threshold change the order of sums only."""
+    import polar_b200 as pg
+    from polar_b200 import autotune
+    n = 4000
+    E = chung_lu(n, 8.0, 2.1, 21, min_degree=1)
+    G = pg.Graph(n, E, 2e-2)
+    op = pg.Op(G)
+    assert np.diff(G._indptr_h).max() > 100  # chunked at two of the thresholds
+    rng = np.random.default_rng(5)
+    W, tau, act = rng.normal(size=(n, R)), np.array([0.0, 0.3, 20.0]), np.sort(rng.permutation(n)[:700])
+    tol, bound = BOUND[prec]
+    with _phases() as seen:
+        X, h, _ = pg.msolve(op, W, tau, act, tol, track=True, precision=prec)
+        for lanes in (16, 32, 64):
+            for sell in (0, 1):
+                for thresh in (16, 100, 5000):
+                    autotune.record(G, prec, R, (lanes, sell, thresh))
+                    X2, h2, _ = pg.msolve(op, W, tau, act, tol, track=True, precision=prec)
+                    assert float((X2 - X).double().norm() / X.double().norm()) < bound, (lanes, sell, thresh)
+                    assert float(((h2 - h).abs() / h).max()) < bound, (lanes, sell, thresh)
+    assert seen["cluster"] == 0 and seen["spmm"] > 0

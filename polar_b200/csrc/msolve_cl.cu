@@ -1174,7 +1174,7 @@ size_t cl_graph_layout(const polar_graph* g, int nA, char* base, ClGraph* C) {
 // them with added edges.  Cluster: its fixed part (more with several CTAs), gathers, the CTA's
 // rows (dearer when their vectors come from L2), the deferred update, the direction's exchange,
 // added edges; as often as its clusters need turns.  Kernels per phase: launches, reductions and
-// gather latency, their vectors, and mk_added's launch or the SpMM's tail.  Of the solves 98.5 %
+// gather latency, their vectors, and mk_added's launch or the SpMM's tail.  Of the solves 98.4 %
 // end up with the faster driver to 3 % (worst 1.27x); without terms for added edges 3 % of them
 // took the cluster solver though it was slower, by up to 1.7x (n = 28,000 R = 64 FP64 with 2,500
 // edges: 113 us an iteration, 82 by phases).

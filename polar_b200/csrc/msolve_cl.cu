@@ -1170,14 +1170,14 @@ size_t cl_graph_layout(const polar_graph* g, int nA, char* base, ClGraph* C) {
 }
 
 // Which driver is the faster one, from clocks per iteration of either, fitted (least squares of the
-// ratio) to 8,700 solves of 1,500 to 58,000 rows with 4 to 18 neighbours, 1 to 128 columns, half of
+// ratio) to 8,700 solves of 1,500 to 58,000 rows with 4 to 18 neighbours, 1 to 128 columns, 44 % of
 // them with added edges.  Cluster: its fixed part (more with several CTAs), gathers, the CTA's
 // rows (dearer when their vectors come from L2), the deferred update, the direction's exchange,
 // added edges; as often as its clusters need turns.  Kernels per phase: launches, reductions and
 // gather latency, their vectors, and mk_added's launch or the SpMM's tail.  Of the solves 98.4 %
 // end up with the faster driver to 3 % (worst 1.27x); without terms for added edges 3 % of them
-// took the cluster solver though it was slower, by up to 1.7x (n = 28,000 R = 64 FP64 with 2,500
-// edges: 113 us an iteration, 82 by phases).
+// took the cluster solver though it was slower, by up to 1.7x (n = 28,000 R = 64 FP64 with added
+// edges in 3,900 rows: 113 us an iteration, 82 by phases).
 template <typename T>
 static bool cl_faster(const ClShape& S) {
   const ClPlan b = cl_plan<T>(S);
